@@ -139,6 +139,19 @@ struct Solve {
     return HPLB_OK;
   }
 
+  // The panel of rows [r0, n) x columns [c0, c0 + jb) as one launch where a
+  // cluster holds it (linv not null: its row map and L11^-1 as well).
+  hplb_status fused(int r0, int c0, int jb, double* dinv, double* linv, int* permU, bool* did) {
+    hplb_ctx* ctx = this->ctx;
+    *did          = false;
+    if(ctx->leaf_kind != HPLB_LEAF_AUTO) return HPLB_OK;
+    CK(launch_panel_fused<double>(A, ld, r0, c0, n, jb, std::max(algo->nbmin, 1),
+                                  std::max(algo->ndiv, 2), algo->rfact, ctx->d_ipiv,
+                                  ctx->d_status, dinv, linv, permU, ctx->s_pan, &ctx->launches,
+                                  did));
+    return HPLB_OK;
+  }
+
   // Factor panel j on the panel stream and build its row map and diagonal
   // inverses; records `done` when finished.
   hplb_status panel(int j, int set, cudaEvent_t done) {
@@ -146,14 +159,18 @@ struct Solve {
     const int   jb  = std::min(algo->nb, n - j);
     cudaEvent_t e0  = next_event(ctx), e1 = next_event(ctx);
     CK(cudaEventRecord(e0, ctx->s_pan));
-    hplb_status s = rpanel(j, j, jb, j, jb);
+    bool        did = false;
+    hplb_status s = fused(j, j, jb, ctx->d_dinv[set], ctx->d_linv[set], ctx->d_perm[set], &did);
     if(s != HPLB_OK) return s;
-    CK(launch_perm(ctx->d_ipiv + j, j, jb, ctx->d_perm[set], ctx->s_pan));
-    CK(launch_diag_inv(A, ld, j, j, jb, ctx->d_dinv[set], ctx->s_pan));
-    ctx->launches += 2;
-    CK(launch_unit_lower_inverse(a(j, j), ld, jb, ctx->d_dinv[set], ctx->d_linv[set], jb,
-                                 ctx->s_pan));
-    ctx->launches += 2;
+    if(!did) {
+      if((s = rpanel(j, j, jb, j, jb)) != HPLB_OK) return s;
+      CK(launch_perm(ctx->d_ipiv + j, j, jb, ctx->d_perm[set], ctx->s_pan));
+      CK(launch_diag_inv(A, ld, j, j, jb, ctx->d_dinv[set], ctx->s_pan));
+      ctx->launches += 2;
+      CK(launch_unit_lower_inverse(a(j, j), ld, jb, ctx->d_dinv[set], ctx->d_linv[set], jb,
+                                   ctx->s_pan));
+      ctx->launches += 1;
+    }
     CK(cudaEventRecord(e1, ctx->s_pan));
     CK(cudaEventRecord(done, ctx->s_pan));
     panel_ev.emplace_back(e0, e1);
@@ -516,7 +533,9 @@ hplb_status hplb_panel_factor(hplb_ctx* ctx, const hplb_algo* algo, int n, int j
   ctx->launches = 0;
   CK(cudaMemsetAsync(ctx->d_status, 0, ST_COUNT * sizeof(int), ctx->s_pan));
   Solve S{ctx, algo, dA, ld, n, {}, {}, {}};
-  if((s = S.rpanel(j, lc, jb, lc, jb)) != HPLB_OK) return s;
+  bool did = false;
+  if((s = S.fused(j, lc, jb, ctx->d_dinv[0], nullptr, nullptr, &did)) != HPLB_OK) return s;
+  if(!did && (s = S.rpanel(j, lc, jb, lc, jb)) != HPLB_OK) return s;
   CK(cudaMemcpyAsync(d_ipiv, ctx->d_ipiv + lc, (size_t)jb * sizeof(int),
                      cudaMemcpyDeviceToDevice, ctx->s_pan));
   CK(cudaStreamSynchronize(ctx->s_pan));

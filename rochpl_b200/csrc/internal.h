@@ -52,6 +52,15 @@ cudaError_t launch_leaf(T* A, int64_t ld, int r0, int end, int c0, int w, int pc
 template <typename T>
 cudaError_t launch_panel_swap(T* A, int64_t ld, const int* ipiv, int r0, int c0, int w, int pc,
                               int pw, cudaStream_t stream);
+// A whole panel by cluster launches (panel_fused.cu): the recursion over
+// columns [c0, c0 + jb) and rows [r0, n), pivots to ipiv[c0 ..], and, when linv
+// is not null, the row map (permU, 2 jb ints) and L11^-1 (jb x jb).  dinv:
+// (jb / 32 + 1) 32 x 32 blocks of scratch.  *done stays false, with nothing
+// launched, for panels it does not hold (too tall, NB or NBMIN too wide).
+template <typename T>
+cudaError_t launch_panel_fused(T* A, int64_t ld, int r0, int c0, int n, int jb, int nbmin,
+                               int ndiv, int rfact, int* ipiv, int* status, T* dinv, T* linv,
+                               int* permU, cudaStream_t stream, int* launches, bool* done);
 cudaError_t launch_perm(const int* ipiv, int ia, int jb, int* permU, cudaStream_t stream);
 template <typename T>
 cudaError_t launch_diag_inv(const T* A, int64_t ld, int r0, int c0, int n, T* inv,
@@ -72,7 +81,7 @@ template <typename T>
 cudaError_t launch_trsm_node(T* A, int64_t ld, int ia, int jb, int lc, T* dinv_scratch, int c0,
                              int n, cudaStream_t stream, int* launches);
 // Linv (jb x jb, leading dimension ldinv) = L^-1 for the unit-lower L at L
-// (leading dimension ldl), by the blocked substitution applied to the identity.
+// (leading dimension ldl) from its 32 x 32 diagonal inverses dinv (panel_fused.cu).
 template <typename T>
 cudaError_t launch_unit_lower_inverse(const T* L, int64_t ldl, int jb, const T* dinv, T* Linv,
                                       int64_t ldinv, cudaStream_t stream);

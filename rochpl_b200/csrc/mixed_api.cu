@@ -111,12 +111,21 @@ struct Mixed {
     st = ctx->s_pan;
     cudaEvent_t p0 = next_event(ctx), p1 = next_event(ctx);
     CK(cudaEventRecord(p0, st));
-    if((s = rpanel(j, j, jb, j, jb)) != HPLB_OK) return s;
-    CK(launch_perm(ctx->d_ipiv + j, j, jb, perm(p), st));
-    CK(launch_diag_inv<float>(W, ldw, j, j, jb, dinv(), st));
-    CK(launch_unit_lower_inverse<float>(w(j, j), ldw, jb, dinv(), linv(p), jb, st));
+    bool did = false;
+    if(ctx->leaf_kind == HPLB_LEAF_AUTO)
+      CK(launch_panel_fused<float>(W, ldw, j, j, n, jb, std::max(algo->nbmin, 1),
+                                   std::max(algo->ndiv, 2), algo->rfact, ctx->d_ipiv,
+                                   ctx->d_status, dinv(), linv(p), perm(p), st,
+                                   &ctx->launches, &did));
+    if(!did) {
+      if((s = rpanel(j, j, jb, j, jb)) != HPLB_OK) return s;
+      CK(launch_perm(ctx->d_ipiv + j, j, jb, perm(p), st));
+      CK(launch_diag_inv<float>(W, ldw, j, j, jb, dinv(), st));
+      CK(launch_unit_lower_inverse<float>(w(j, j), ldw, jb, dinv(), linv(p), jb, st));
+      ctx->launches += 3;
+    }
     CK(launch_upper_inverse(jb, w(j, j), ldw, uinv(p), upper_work(), dinv_piece(), st));
-    ctx->launches += 9;
+    ctx->launches += 4;
     CK(cudaEventRecord(p1, st));
     CK(cudaEventRecord(done, st));
     panel_ev.emplace_back(p0, p1);
