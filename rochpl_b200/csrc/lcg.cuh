@@ -33,20 +33,17 @@ __host__ __device__ inline Jump jump_by(uint64_t k) {
 
 __host__ __device__ inline uint64_t apply(Jump j, uint64_t x) { return j.a * x + j.c; }
 
-// Matrix entry from a state, with the reference's operation order
-// (src/matgen/HPL_pdrandmat_device.cpp:65-73).  Every multiply or divide is by
-// a power of two and therefore exact; the explicit _rn intrinsics keep the two
-// rounded additions and the final subtraction from being contracted.
+// Matrix entry from a state.  The reference adds the four 16-bit parts with
+// power-of-two scales (src/matgen/HPL_pdrandmat_device.cpp:65-73); of its steps
+// only two round: t = RN(hi + lo 2^-32) of the state's 32-bit halves (the sums
+// before it have at most 48 bits) and RN(0.5 - t 2^-32).  Two fused multiply-
+// adds round at the same places.  The halves become doubles by their bits
+// (2^52 + v) - 2^52 instead of four integer conversions (hplb_matgen at
+// N = 16384: 620 -> 533 us).
 __device__ __forceinline__ double lcg_value(uint64_t r) {
-  const double p1 = (double)(uint32_t)(r & 65535ull);
-  const double p2 = (double)(uint32_t)((r >> 16) & 65535ull);
-  const double p3 = (double)(uint32_t)((r >> 32) & 65535ull);
-  const double p4 = (double)(uint32_t)((r >> 48) & 65535ull);
-  double t = __dadd_rn(p1, __dmul_rn(p2, 65536.0));
-  t        = __dmul_rn(__dmul_rn(t, 0x1p-31), 0.5);
-  t        = __dadd_rn(t, p3);
-  t        = __dadd_rn(t, __dmul_rn(p4, 65536.0));
-  return __dsub_rn(0.5, __dmul_rn(__dmul_rn(t, 0x1p-31), 0.5));
+  const double hi = __hiloint2double(0x43300000, (int)(uint32_t)(r >> 32)) - 0x1p52;
+  const double lo = __hiloint2double(0x43300000, (int)(uint32_t)r) - 0x1p52;
+  return __fma_rn(__fma_rn(lo, 0x1p-32, hi), -0x1p-32, 0.5);
 }
 
 }  // namespace hplb

@@ -957,37 +957,54 @@ HPLB_DEV void gemm_tiles(int m, int n, int k, const float* A, int64_t lda, const
     }
 }
 
-// A 64 x 64 tile of the products below by a CTA: sign * sum over k in [k0, k1)
+// FP64: a 16 x 32 tile of the products below for a warp, straight from L2 by
+// DMMA: acc = sum over k in [k0, k1) of A(r, k) B(k, c), A column-major, B by its
+// two strides; then out(r, c) = sign * acc at out[r sr + c sc].
+HPLB_DEV void tri_warp(const double* A, int64_t lda, int mr, const double* B, int64_t sbk,
+                       int64_t sbn, int nc, int k0, int k1, double* out, int64_t sr, int64_t sc,
+                       double sign) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  double    acc[4][4];
+#pragma unroll
+  for(int j = 0; j < 4; ++j)
+#pragma unroll
+    for(int r = 0; r < 4; ++r) acc[j][r] = 0.0;
+#pragma unroll 4
+  for(int k = k0; k < k1; k += 8) {
+    double a[4], b[4][2];
+#pragma unroll
+    for(int r = 0; r < 4; ++r) {
+      const int rr = g + (r & 1) * 8, kk = k + t4 + (r >> 1) * 4;
+      a[r] = (rr < mr && kk < k1) ? __ldcg(A + (size_t)rr + (size_t)kk * lda) : 0.0;
+    }
+#pragma unroll
+    for(int j = 0; j < 4; ++j)
+#pragma unroll
+      for(int h = 0; h < 2; ++h) {
+        const int cc = j * 8 + g, kk = k + t4 + h * 4;
+        b[j][h] = (cc < nc && kk < k1) ? __ldcg(B + (size_t)kk * sbk + (size_t)cc * sbn) : 0.0;
+      }
+#pragma unroll
+    for(int j = 0; j < 4; ++j) dmma(acc[j], a, b[j]);
+  }
+#pragma unroll
+  for(int j = 0; j < 4; ++j)
+#pragma unroll
+    for(int r = 0; r < 4; ++r) {
+      const int rr = g + (r >> 1) * 8, cc = j * 8 + 2 * t4 + (r & 1);
+      if(rr < mr && cc < nc) out[(size_t)rr * sr + (size_t)cc * sc] = sign * acc[j][r];
+    }
+}
+
+// FP32: a 64 x 64 tile by a CTA: sign * sum over k in [k0, k1)
 // of A(r, k) B(k, c) to out[r sr + c sc], for r < mr and c < nc.  A column-major,
 // B by its two strides (one of them 1); k-slices of 32 through two cp.async
 // buffers (the triangular factor, B in step 0 and A in step 1, with its tile at
 // row or column `at`: what stands above its diagonal blocks is not its own and
-// counts as 0), A in k-rows of pitch 68, B in columns of pitch 36 (= 4 mod 16: free of
-// conflicts for the FP64 fragments).
+// counts as 0).
 constexpr int kTriTile = 64, kTriK = 32, kTriPa = kTriTile + 4, kTriPb = kTriK + 4;
 constexpr int kTriStage = kTriK * kTriPa + kTriTile * kTriPb;  // elements of a buffer
 
-HPLB_DEV void tri_step(double (&acc)[16], const double* as, const double* bs) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
-  const int r0 = (warp & 3) * 16 + g, c0 = (warp >> 2) * 32 + g;
-#pragma unroll
-  for(int k = 0; k < kTriK; k += 8) {
-    const double* pa   = as + (k + t4) * kTriPa + r0;
-    const double  a[4] = {pa[0], pa[8], pa[4 * kTriPa], pa[4 * kTriPa + 8]};
-#pragma unroll
-    for(int j = 0; j < 4; ++j) {
-      const double* pb   = bs + (c0 + 8 * j) * kTriPb + k + t4;
-      const double  b[2] = {pb[0], pb[4]};
-      dmma(*reinterpret_cast<double(*)[4]>(&acc[4 * j]), a, b);
-    }
-  }
-}
-HPLB_DEV int tri_row(double, int e) {
-  return ((threadIdx.x >> 5) & 3) * 16 + ((threadIdx.x & 31) >> 2) + ((e >> 1) & 1) * 8;
-}
-HPLB_DEV int tri_col(double, int e) {
-  return (threadIdx.x >> 7) * 32 + (e >> 2) * 8 + 2 * (threadIdx.x & 3) + (e & 1);
-}
 HPLB_DEV void tri_step(float (&acc)[16], const float* as, const float* bs) {
   const int ty = threadIdx.x % 16, tx = threadIdx.x / 16;
 #pragma unroll 2
@@ -1010,21 +1027,17 @@ HPLB_DEV void tri_step(float (&acc)[16], const float* as, const float* bs) {
     }
   }
 }
-HPLB_DEV int tri_row(float, int e) { return threadIdx.x % 16 * 4 + (e & 3); }
-HPLB_DEV int tri_col(float, int e) { return threadIdx.x / 16 * 4 + (e >> 2); }
-
-template <typename T>
-HPLB_DEV void tri_tile(const T* A, int64_t lda, int mr, const T* B, int64_t sbk, int64_t sbn,
-                       int nc, int k0, int k1, int step, int at, T* out, int64_t sr, int64_t sc,
-                       T sign, T* sm) {
-  auto load = [&](int kb, T* st) {
+HPLB_DEV void tri_tile(const float* A, int64_t lda, int mr, const float* B, int64_t sbk, int64_t sbn,
+                       int nc, int k0, int k1, int step, int at, float* out, int64_t sr, int64_t sc,
+                       float sign, float* sm) {
+  auto load = [&](int kb, float* st) {
 #pragma unroll
     for(int h = 0; h < kTriTile * kTriK / kThreads; ++h) {
       const int  e = threadIdx.x + h * kThreads, r = e % kTriTile, k = e / kTriTile;
       const bool in = r < mr && kb + k < k1 && (step == 0 || kb + k < at + r / kTri * kTri + kTri);
       cp_async1(s_addr(st + k * kTriPa + r), in ? A + (size_t)r + (size_t)(kb + k) * lda : A, in);
     }
-    T* sb = st + kTriK * kTriPa;
+    float* sb = st + kTriK * kTriPa;
 #pragma unroll
     for(int h = 0; h < kTriTile * kTriK / kThreads; ++h) {
       const int  e = threadIdx.x + h * kThreads;
@@ -1035,9 +1048,9 @@ HPLB_DEV void tri_tile(const T* A, int64_t lda, int mr, const T* B, int64_t sbk,
     }
     cp_commit();
   };
-  T acc[16];
+  float acc[16];
 #pragma unroll
-  for(int e = 0; e < 16; ++e) acc[e] = (T)0;
+  for(int e = 0; e < 16; ++e) acc[e] = 0.f;
   load(k0, sm);
   int buf = 0;
   for(int kb = k0; kb < k1; kb += kTriK, buf ^= 1) {
@@ -1052,7 +1065,7 @@ HPLB_DEV void tri_tile(const T* A, int64_t lda, int mr, const T* B, int64_t sbk,
   }
 #pragma unroll
   for(int e = 0; e < 16; ++e) {
-    const int r = tri_row(T(0), e), c = tri_col(T(0), e);
+    const int r = threadIdx.x % 16 * 4 + (e & 3), c = threadIdx.x / 16 * 4 + (e >> 2);
     if(r < mr && c < nc) out[(size_t)r * sr + (size_t)c * sc] = sign * acc[e];
   }
 }
@@ -1060,8 +1073,8 @@ HPLB_DEV void tri_tile(const T* A, int64_t lda, int mr, const T* B, int64_t sbk,
 // X (jb x jb, leading dimension ldx) = L^-1 for the unit-lower L at L, from its
 // inverted 32 x 32 diagonal blocks, by doubling: for neighbouring blocks of s
 // columns, [A 0; B C]^-1 = [A^-1 0; -C^-1 B A^-1, C^-1], each product a tile per
-// CTA (a 16 x 32 tile per warp straight from L2 took 2.5 times as long at jb =
-// 512: the operands crossed to the SMs four times as often).  log2(jb / 32) levels of two products and two cluster barriers instead
+// warp (FP64) or CTA (FP32, whose FFMA loop wants its operands in shared memory:
+// 197 us at jb = 512 with warp tiles, 68 with these).  log2(jb / 32) levels of two products and two cluster barriers instead
 // of a chain of jb / 32 substitution steps, which the blocked substitution on
 // the identity needs.  B A^-1 waits, transposed, in X's block above the diagonal.
 template <typename T>
@@ -1076,22 +1089,33 @@ HPLB_DEV void lower_inverse(const T* L, int64_t ldl, int jb, const T* dinv, T* X
           __ldcg(dinv + (size_t)(c / kTri) * kTri * kTri + (c % kTri) * kTri + lane);
   }
   for(int s = kTri; s < jb; s *= 2) {
-    const int t = (s + kTriTile - 1) / kTriTile, units = (jb + 2 * s - 1) / (2 * s) * t * t;
+    constexpr bool wide = sizeof(T) == 4;
+    constexpr int  TR = wide ? kTriTile : 16, TC = wide ? kTriTile : 32;
+    const int      tr = (s + TR - 1) / TR, tc = (s + TC - 1) / TC;
+    const int      units = (jb + 2 * s - 1) / (2 * s) * tr * tc;
     for(int step = 0; step < 2; ++step) {
       cluster_sync();
-      for(int e = (int)me; e < units; e += (int)G) {
-        const int base = e / (t * t) * 2 * s, r = e / t % t * kTriTile, c = e % t * kTriTile;
+      for(int e = wide ? (int)me : gw; e < units; e += wide ? (int)G : nw) {
+        const int base = e / (tr * tc) * 2 * s, r = e / tc % tr * TR, c = e % tc * TC;
         const int s2 = min(s, jb - base - s), mr = s2 - r;
         if(mr <= 0) continue;
-        T* bt = X + (size_t)base + (size_t)(base + s) * ldx;  // (B A^-1)^T
-        if(step == 0)
-          tri_tile<T>(L + (size_t)(base + s + r) + (size_t)base * ldl, ldl, mr,
-                      X + (size_t)base + (size_t)(base + c) * ldx, 1, ldx, s - c, c, s, 0, c,
-                      bt + (size_t)c + (size_t)r * ldx, ldx, 1, (T)1, sm);
+        T*       bt = X + (size_t)base + (size_t)(base + s) * ldx;  // (B A^-1)^T
+        const T* A  = step == 0 ? L + (size_t)(base + s + r) + (size_t)base * ldl
+                                : X + (size_t)(base + s + r) + (size_t)(base + s) * ldx;
+        const T* B  = step == 0 ? X + (size_t)base + (size_t)(base + c) * ldx : bt + c;
+        T* out = step == 0 ? bt + (size_t)c + (size_t)r * ldx
+                           : X + (size_t)(base + s + r) + (size_t)(base + c) * ldx;
+        const int64_t lda = step == 0 ? ldl : ldx, sbk = step == 0 ? 1 : ldx,
+                      sbn = step == 0 ? ldx : 1;
+        // The triangular factor's columns from the tile's on, rows up to its last.
+        const int k0 = step == 0 ? c / kTri * kTri : 0;
+        const int k1 = step == 0 ? s : min(s2, (r + TR + kTri - 1) / kTri * kTri);
+        const T   sign = step == 0 ? (T)1 : (T)-1;
+        if constexpr(wide)
+          tri_tile(A, lda, mr, B, sbk, sbn, s - c, k0, k1, step, step == 0 ? c : r, out, sbn, sbk,
+                   sign, sm);
         else
-          tri_tile<T>(X + (size_t)(base + s + r) + (size_t)(base + s) * ldx, ldx, mr, bt + c, ldx,
-                      1, s - c, 0, min(s2, r + kTriTile), 1, r,
-                      X + (size_t)(base + s + r) + (size_t)(base + c) * ldx, 1, ldx, (T)-1, sm);
+          tri_warp(A, lda, mr, B, sbk, sbn, s - c, k0, k1, out, sbn, sbk, sign);
       }
     }
   }
@@ -1114,7 +1138,7 @@ constexpr size_t dyn_bytes() {
   b = at_least(b, (size_t)GemmCfg<T>::stages(1) * GemmCfg<T>::stage(1) * sizeof(T));
   b = at_least(b, (size_t)GemmCfg<T>::stages(2) * GemmCfg<T>::stage(2) * sizeof(T));
   b = at_least(b, (size_t)GemmCfg<T>::stages(4) * GemmCfg<T>::stage(4) * sizeof(T));
-  b = at_least(b, (size_t)2 * kTriStage * sizeof(T));
+  b = at_least(b, (size_t)2 * kTriStage * sizeof(float));
   b = at_least(b, (size_t)kWarps * 2 * (kMaxNb + 1) * sizeof(T));           // trsm_cols<T, 2>
   return at_least(b, (size_t)kWarps * kTri * kTopPitch * sizeof(T));        // invert_blocks
 }
@@ -1400,7 +1424,7 @@ cudaError_t launch_unit_lower_inverse(const T* L, int64_t ldl, int jb, const T* 
   static signed char placeable[kMaxG + 1] = {};
   for(int g = cluster_for((jb + 31) / 32); g > 0; g /= 2) {
     bool              done = false;
-    const cudaError_t e    = launch_cluster(lower_inverse_kernel<T>, g, 2 * kTriStage * sizeof(T),
+    const cudaError_t e    = launch_cluster(lower_inverse_kernel<T>, g, 2 * kTriStage * sizeof(float),
                                             placeable, stream, &done,
                                             L, ldl, jb, dinv, Linv, ldinv);
     if(done || e != cudaSuccess) return e;

@@ -23,6 +23,9 @@ namespace {
 
 constexpr int kRowThreads = 256;
 constexpr int kChunk      = 2048;  // columns per partial sum
+// The stored-matrix pass (rows_cols_partial): columns whose sums wait in shared
+// memory before they leave a CTA.
+constexpr int kPassHalf = 512;
 
 struct ResTabs {
   Jump pow2[64];
@@ -41,15 +44,15 @@ HPLB_DEV uint64_t state_of(const ResTabs& T, uint64_t k) {
 template <bool LCG>
 __global__ void __launch_bounds__(kRowThreads)
 rows_partial(int n, const double* __restrict__ A, int64_t ld, const double* __restrict__ X,
-             const ResTabs* __restrict__ T, double* part_r, double* part_a) {
+             const __grid_constant__ ResTabs T, double* part_r, double* part_a) {
   const int i  = blockIdx.x * kRowThreads + threadIdx.x;
   const int j0 = blockIdx.y * kChunk;
   const int j1 = min(n, j0 + kChunk);
   if(i >= n) return;
   double acc = 0.0, asum = 0.0;
   if(LCG) {
-    const Jump cj = T->col;
-    uint64_t   s  = state_of(*T, (uint64_t)i + (uint64_t)j0 * (uint64_t)n);
+    const Jump cj = T.col;
+    uint64_t   s  = state_of(T, (uint64_t)i + (uint64_t)j0 * (uint64_t)n);
     for(int j = j0; j < j1; ++j) {
       const double a = lcg_value(s);
       acc += a * X[j];
@@ -67,6 +70,67 @@ rows_partial(int n, const double* __restrict__ A, int64_t ld, const double* __re
   }
   part_r[(size_t)blockIdx.y * n + i] = acc;
   part_a[(size_t)blockIdx.y * n + i] = asum;
+}
+
+// Row sums of A x and |A| and column sums of |A| in one read of the stored A:
+// HBM-bound, and a second read for the column sums would double it.  A column's
+// sum over a warp's 32 rows is folded 16 columns at a time: in each of 4 steps a
+// lane hands half of its columns to its partner, the last step adds neighbours
+// (16 exchanges for 16 columns); the warps' sums meet in shared memory, the
+// CTAs' in part_c (a row of n per 256 rows of A).  Four CTAs per SM, so that one's
+// folding runs under the others' loads: the whole check at N = 16384 takes 480 us
+// (858 with two passes, 725 with 32 columns at a time and two CTAs).  col_sums adds in the same order, so the
+// stored and the regenerated check agree to the last bit.
+__global__ void __launch_bounds__(kRowThreads, 4)
+rows_cols_partial(int n, const double* __restrict__ A, int64_t ld, const double* __restrict__ X,
+                  double* part_r, double* part_a, double* part_c) {
+  constexpr int     kW = kRowThreads / 32, kU = 16;
+  __shared__ double sc[kW][kPassHalf];
+  const int     lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int     i = blockIdx.x * kRowThreads + threadIdx.x;
+  const bool    in = i < n;
+  const int     jb = blockIdx.y * kChunk, je = min(n, jb + kChunk);
+  const double* a = A + (in ? i : 0);
+  double        acc = 0.0, asum = 0.0;
+  for(int jh = jb; jh < je; jh += kPassHalf) {
+    const int jhe = min(je, jh + kPassHalf);
+    for(int j = jh; j < jhe; j += kU) {
+      double c[kU];
+#pragma unroll
+      for(int u = 0; u < kU; ++u)
+        c[u] = in && j + u < jhe ? __ldcs(a + (size_t)(j + u) * (size_t)ld) : 0.0;
+#pragma unroll
+      for(int u = 0; u < kU; ++u) {
+        if(j + u < jhe) acc += c[u] * X[j + u];
+        c[u] = fabs(c[u]);
+        asum += c[u];
+      }
+#pragma unroll
+      for(int s = kU / 2; s > 0; s >>= 1) {
+        const bool up = (lane & (2 * s)) != 0;
+#pragma unroll
+        for(int u = 0; u < kU / 2; ++u)
+          if(u < s) {
+            const double give = up ? c[u] : c[u + s], keep = up ? c[u + s] : c[u];
+            c[u]              = keep + __shfl_xor_sync(0xffffffffu, give, 2 * s);
+          }
+      }
+      c[0] += __shfl_xor_sync(0xffffffffu, c[0], 1);
+      if((lane & 1) == 0) sc[warp][j - jh + (lane >> 1)] = c[0];  // column j + lane / 2
+    }
+    __syncthreads();
+    for(int j = threadIdx.x; j < jhe - jh; j += kRowThreads) {
+      double t = 0.0;
+#pragma unroll
+      for(int w = 0; w < kW; ++w) t += sc[w][j];
+      part_c[(size_t)blockIdx.x * n + jh + j] = t;
+    }
+    __syncthreads();
+  }
+  if(in) {
+    part_r[(size_t)blockIdx.y * n + i] = acc;
+    part_a[(size_t)blockIdx.y * n + i] = asum;
+  }
 }
 
 HPLB_DEV double block_max(double v, double* sh) {
@@ -96,7 +160,7 @@ HPLB_DEV double block_sum(double v, double* sh) {
 template <bool LCG>
 __global__ void __launch_bounds__(kRowThreads)
 rows_final(int n, int nch, const double* __restrict__ A, int64_t ld, const double* __restrict__ X,
-           const ResTabs* __restrict__ T, const double* part_r, const double* part_a,
+           const __grid_constant__ ResTabs T, const double* part_r, const double* part_a,
            double* blk) {
   __shared__ double sh[32];
   const int i = blockIdx.x * kRowThreads + threadIdx.x;
@@ -104,7 +168,7 @@ rows_final(int n, int nch, const double* __restrict__ A, int64_t ld, const doubl
   if(i < n) {
     double b;
     if(LCG)
-      b = lcg_value(state_of(*T, (uint64_t)i + (uint64_t)n * (uint64_t)n));
+      b = lcg_value(state_of(T, (uint64_t)i + (uint64_t)n * (uint64_t)n));
     else
       b = A[(size_t)i + (size_t)n * ld];
     double acc = 0.0;
@@ -132,27 +196,38 @@ rows_final(int n, int nch, const double* __restrict__ A, int64_t ld, const doubl
   }
 }
 
-template <bool LCG>
+// The largest column sum of a CTA's 256 columns, from the nrg row groups' sums.
 __global__ void __launch_bounds__(256)
-col_sums(int n, const double* __restrict__ A, int64_t ld, const ResTabs* __restrict__ T,
-         double* blkc) {
+col_max(int n, int nrg, const double* __restrict__ part_c, double* blkc) {
+  __shared__ double sh[32];
+  const int j = blockIdx.x * 256 + threadIdx.x;
+  double    s = 0.0;
+  if(j < n)
+    for(int g = 0; g < nrg; ++g) s += part_c[(size_t)g * n + j];
+  const double m = block_max(s, sh);
+  if(threadIdx.x == 0) blkc[blockIdx.x] = m;
+}
+
+// Column sums of the regenerated matrix.
+__global__ void __launch_bounds__(256)
+col_sums(int n, const __grid_constant__ ResTabs T, double* blkc) {
   __shared__ double sh[32];
   const int lane = threadIdx.x & 31;
   const int j    = blockIdx.x * 8 + (threadIdx.x >> 5);
   double    s    = 0.0;
   if(j < n) {
-    if(LCG) {
-      const Jump st = T->step32;
-      uint64_t   x  = state_of(*T, (uint64_t)lane + (uint64_t)j * (uint64_t)n);
-      for(int i = lane; i < n; i += 32) {
-        s += fabs(lcg_value(x));
-        x = apply(st, x);
+    const Jump st = T.step32;
+    uint64_t   x  = state_of(T, (uint64_t)lane + (uint64_t)j * (uint64_t)n);
+    for(int i0 = 0; i0 < n; i0 += kRowThreads) {
+      double t = 0.0;
+      for(int i = i0 + lane; i - lane < min(n, i0 + kRowThreads); i += 32) {
+        double v = i < n ? fabs(lcg_value(x)) : 0.0;
+        x        = apply(st, x);
+        for(int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+        t += v;
       }
-    } else {
-      const double* a = A + (size_t)j * ld;
-      for(int i = lane; i < n; i += 32) s += fabs(a[i]);
+      s += t;
     }
-    for(int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
   }
   // s valid in lane 0 of each warp; block max over the 8 columns.
   s = __shfl_sync(0xffffffffu, s, 0);
@@ -194,30 +269,10 @@ __global__ void __launch_bounds__(256) finish(int n, int nrb, int ncb, const dou
   }
 }
 
-}  // namespace
-
-size_t residual_ws_doubles(int n) {
-  const size_t nch = (size_t)(n + kChunk - 1) / kChunk;
-  const size_t nrb = (size_t)(n + kRowThreads - 1) / kRowThreads;
-  const size_t ncb = (size_t)(n + 7) / 8;
-  const size_t tabs = (sizeof(ResTabs) + 7) / 8;
-  return 2 * nch * (size_t)n + 5 * nrb + ncb + tabs + 16;
-}
-
-cudaError_t launch_residual(int n, const double* A, int64_t ld, bool lcg, uint64_t seed,
-                            const double* X, double* ws, double* out8, cudaStream_t stream) {
-  if(n <= 0) return cudaMemsetAsync(out8, 0, 8 * sizeof(double), stream);
-  const int nch = (n + kChunk - 1) / kChunk;
-  const int nrb = (n + kRowThreads - 1) / kRowThreads;
-  const int ncb = (n + 7) / 8;
-  double* part_r = ws;
-  double* part_a = part_r + (size_t)nch * n;
-  double* blk    = part_a + (size_t)nch * n;
-  double* blkc   = blk + (size_t)nrb * 5;
-  ResTabs* dT = reinterpret_cast<ResTabs*>(((uintptr_t)(blkc + ncb) + 63) & ~(uintptr_t)63);
-
+// The LCG jumps of an n-row matrix, passed to the kernels by value.
+ResTabs make_tabs(int n, uint64_t seed) {
   ResTabs T;
-  Jump p{kLcgMult, kLcgAdd};
+  Jump    p{kLcgMult, kLcgAdd};
   for(int b = 0; b < 64; ++b) {
     T.pow2[b] = p;
     p         = compose(p, p);
@@ -225,22 +280,50 @@ cudaError_t launch_residual(int n, const double* A, int64_t ld, bool lcg, uint64
   T.col    = jump_by((uint64_t)n);
   T.step32 = jump_by(32);
   T.x1     = kLcgMult * seed + kLcgAdd;
-  cudaError_t e = cudaMemcpyAsync(dT, &T, sizeof(T), cudaMemcpyHostToDevice, stream);
-  if(e != cudaSuccess) return e;
-  // The host copy of T must outlive the async copy.
-  e = cudaStreamSynchronize(stream);
-  if(e != cudaSuccess) return e;
+  return T;
+}
 
-  dim3 g1(nrb, nch);
-  if(lcg) {
-    rows_partial<true><<<g1, kRowThreads, 0, stream>>>(n, A, ld, X, dT, part_r, part_a);
-    rows_final<true><<<nrb, kRowThreads, 0, stream>>>(n, nch, A, ld, X, dT, part_r, part_a, blk);
-    col_sums<true><<<ncb, 256, 0, stream>>>(n, A, ld, dT, blkc);
-  } else {
-    rows_partial<false><<<g1, kRowThreads, 0, stream>>>(n, A, ld, X, dT, part_r, part_a);
-    rows_final<false><<<nrb, kRowThreads, 0, stream>>>(n, nch, A, ld, X, dT, part_r, part_a, blk);
-    col_sums<false><<<ncb, 256, 0, stream>>>(n, A, ld, dT, blkc);
+}  // namespace
+
+size_t residual_ws_doubles(int n) {
+  const size_t nch = (size_t)(n + kChunk - 1) / kChunk;
+  const size_t nrb = (size_t)(n + kRowThreads - 1) / kRowThreads;
+  const size_t ncb = (size_t)(n + 7) / 8;
+  const size_t tabs = (sizeof(ResTabs) + 7) / 8;
+  return (2 * nch + nrb) * (size_t)n + 5 * nrb + ncb + tabs + 16;
+}
+
+cudaError_t launch_residual(int n, const double* A, int64_t ld, bool lcg, uint64_t seed,
+                            const double* X, double* ws, double* out8, cudaStream_t stream) {
+  if(n <= 0) return cudaMemsetAsync(out8, 0, 8 * sizeof(double), stream);
+  const int nrb = (n + kRowThreads - 1) / kRowThreads;
+  if(!lcg) {
+    const int nch = (n + kChunk - 1) / kChunk;
+    const int ncb = (n + 255) / 256;
+    double*   part_r = ws;
+    double*   part_a = part_r + (size_t)nch * n;
+    double*   part_c = part_a + (size_t)nch * n;
+    double*   blk    = part_c + (size_t)nrb * n;
+    double*   blkc   = blk + (size_t)nrb * 5;
+    rows_cols_partial<<<dim3(nrb, nch), kRowThreads, 0, stream>>>(n, A, ld, X, part_r, part_a,
+                                                                  part_c);
+    rows_final<false><<<nrb, kRowThreads, 0, stream>>>(n, nch, A, ld, X, ResTabs{}, part_r, part_a,
+                                                       blk);
+    col_max<<<ncb, 256, 0, stream>>>(n, nrb, part_c, blkc);
+    finish<<<1, 256, 0, stream>>>(n, nrb, ncb, blk, blkc, out8);
+    return cudaGetLastError();
   }
+  const int nch = (n + kChunk - 1) / kChunk;
+  const int ncb = (n + 7) / 8;
+  double* part_r = ws;
+  double* part_a = part_r + (size_t)nch * n;
+  double* blk    = part_a + (size_t)nch * n;
+  double* blkc   = blk + (size_t)nrb * 5;
+  const ResTabs T = make_tabs(n, seed);
+  dim3 g1(nrb, nch);
+  rows_partial<true><<<g1, kRowThreads, 0, stream>>>(n, A, ld, X, T, part_r, part_a);
+  rows_final<true><<<nrb, kRowThreads, 0, stream>>>(n, nch, A, ld, X, T, part_r, part_a, blk);
+  col_sums<<<ncb, 256, 0, stream>>>(n, T, blkc);
   finish<<<1, 256, 0, stream>>>(n, nrb, ncb, blk, blkc, out8);
   return cudaGetLastError();
 }
@@ -259,28 +342,13 @@ __global__ void rows_sum(int n, int nch, const double* __restrict__ part, double
 // out[i] = A(i, col), from the stored matrix or regenerated from the LCG.
 template <bool LCG>
 __global__ void column_of(int n, int col, const double* __restrict__ A, int64_t ld,
-                          const ResTabs* __restrict__ T, double* __restrict__ out) {
+                          const __grid_constant__ ResTabs T, double* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if(i >= n) return;
   if(LCG)
-    out[i] = lcg_value(state_of(*T, (uint64_t)i + (uint64_t)col * (uint64_t)n));
+    out[i] = lcg_value(state_of(T, (uint64_t)i + (uint64_t)col * (uint64_t)n));
   else
     out[i] = A[(size_t)i + (size_t)col * ld];
-}
-
-cudaError_t upload_tabs(int n, uint64_t seed, ResTabs* dT, cudaStream_t stream) {
-  ResTabs T;
-  Jump p{kLcgMult, kLcgAdd};
-  for(int b = 0; b < 64; ++b) {
-    T.pow2[b] = p;
-    p         = compose(p, p);
-  }
-  T.col    = jump_by((uint64_t)n);
-  T.step32 = jump_by(32);
-  T.x1     = kLcgMult * seed + kLcgAdd;
-  cudaError_t e = cudaMemcpyAsync(dT, &T, sizeof(T), cudaMemcpyHostToDevice, stream);
-  if(e != cudaSuccess) return e;
-  return cudaStreamSynchronize(stream);  // T lives on this stack frame
 }
 
 }  // namespace
@@ -294,15 +362,12 @@ cudaError_t launch_gemv_hpl(int n, const double* A, int64_t ld, bool lcg, uint64
   const int nrb = (n + kRowThreads - 1) / kRowThreads;
   double*   part_r = ws;
   double*   part_a = part_r + (size_t)nch * n;
-  ResTabs*  dT = reinterpret_cast<ResTabs*>(((uintptr_t)(part_a + (size_t)nch * n) + 63) &
-                                            ~(uintptr_t)63);
-  cudaError_t e = upload_tabs(n, seed, dT, stream);
-  if(e != cudaSuccess) return e;
+  const ResTabs T = make_tabs(n, seed);
   dim3 g1(nrb, nch);
   if(lcg)
-    rows_partial<true><<<g1, kRowThreads, 0, stream>>>(n, A, ld, x, dT, part_r, part_a);
+    rows_partial<true><<<g1, kRowThreads, 0, stream>>>(n, A, ld, x, T, part_r, part_a);
   else
-    rows_partial<false><<<g1, kRowThreads, 0, stream>>>(n, A, ld, x, dT, part_r, part_a);
+    rows_partial<false><<<g1, kRowThreads, 0, stream>>>(n, A, ld, x, T, part_r, part_a);
   rows_sum<<<nrb, kRowThreads, 0, stream>>>(n, nch, part_r, y);
   return cudaGetLastError();
 }
@@ -311,14 +376,13 @@ cudaError_t launch_gemv_hpl(int n, const double* A, int64_t ld, bool lcg, uint64
 cudaError_t launch_column_hpl(int n, int col, const double* A, int64_t ld, bool lcg,
                               uint64_t seed, double* out, double* ws, cudaStream_t stream) {
   if(n <= 0) return cudaSuccess;
-  ResTabs* dT = reinterpret_cast<ResTabs*>(((uintptr_t)ws + 63) & ~(uintptr_t)63);
-  cudaError_t e = upload_tabs(n, seed, dT, stream);
-  if(e != cudaSuccess) return e;
+  (void)ws;
+  const ResTabs T = make_tabs(n, seed);
   const int nrb = (n + kRowThreads - 1) / kRowThreads;
   if(lcg)
-    column_of<true><<<nrb, kRowThreads, 0, stream>>>(n, col, A, ld, dT, out);
+    column_of<true><<<nrb, kRowThreads, 0, stream>>>(n, col, A, ld, T, out);
   else
-    column_of<false><<<nrb, kRowThreads, 0, stream>>>(n, col, A, ld, dT, out);
+    column_of<false><<<nrb, kRowThreads, 0, stream>>>(n, col, A, ld, T, out);
   return cudaGetLastError();
 }
 
