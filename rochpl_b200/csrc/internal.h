@@ -62,6 +62,9 @@ cudaError_t launch_panel_fused(T* A, int64_t ld, int r0, int c0, int n, int jb, 
                                int ndiv, int rfact, int* ipiv, int* status, T* dinv, T* linv,
                                int* permU, cudaStream_t stream, int* launches, bool* done);
 cudaError_t launch_perm(const int* ipiv, int ia, int jb, int* permU, cudaStream_t stream);
+// The same for every nb-wide panel of an n-row factorisation in one launch:
+// panel p's map at permU + 2 nb p.
+cudaError_t launch_perm_panels(const int* ipiv, int n, int nb, int* permU, cudaStream_t stream);
 template <typename T>
 cudaError_t launch_diag_inv(const T* A, int64_t ld, int r0, int c0, int n, T* inv,
                             cudaStream_t stream);
@@ -117,6 +120,12 @@ cudaError_t launch_col_rank1(double* A, int64_t ld, int r0, int r1, int c0, int 
 cudaError_t launch_trsm_upper(const double* A, int64_t ld, int n, int nrhs, const double* Y,
                               int64_t ldy, double* X, int64_t ldx, int* flags, int* status,
                               cudaStream_t stream, int* launches);
+// X (rows x nrhs) <- L^-1 X for the unit-lower ns x ns L in the first ns rows, and
+// X -= L21 X_top in the rows - ns below, in one persistent launch per 32
+// right-hand sides; flags: trsv_flag_ints(ns).
+cudaError_t launch_trsm_lower(const double* L, int64_t ldl, int ns, int rows, int nrhs, double* X,
+                              int64_t ldx, int* flags, int* status, cudaStream_t stream,
+                              int* launches);
 cudaError_t launch_gemv_acc(int m, int k, const double* U, int64_t ld, const double* x,
                             double* z, cudaStream_t stream);
 cudaError_t launch_vsub(int n, const double* y, const double* s, double* r, cudaStream_t stream);
@@ -191,10 +200,10 @@ cudaError_t launch_unit_lower_view(int kind, int jb, const double* T, int64_t ld
 cudaError_t launch_rows_xform(int jb, int n, const double* in, int64_t ldi, double* out,
                               int64_t ldo, const double* d, bool flip, bool scale,
                               cudaStream_t st);
-// X (jb x ncols) <- L^-1 X, unit-lower L, for few right-hand sides: one CTA per
-// column (dinv: the 32 x 32 diagonal inverses of L).
-cudaError_t launch_trsm_small(int jb, int ncols, double* X, int64_t ldx, const double* L,
-                              int64_t ldl, const double* dinv, cudaStream_t st);
+// A panel's interchanges (row map permU, 2 jb ints) on rows ia .. of the n columns
+// of X in place.
+cudaError_t launch_permute_rows(double* X, int64_t ldx, int ia, int jb, const int* permU, int n,
+                                cudaStream_t st);
 // C (jb x nrhs) -= M (jb x K) Y (K x nrhs) for K >> jb, nrhs: split-k partial
 // products into ws (splitk_ws_doubles) and a fixed-order reduction.
 size_t      splitk_ws_doubles(int jb, int nrhs, int K);

@@ -823,7 +823,7 @@ panel_swap_kernel(T* A, int64_t ld, const int* ipiv, int r0, int c0, int w, int 
 //   permU[jb + s] = destination of original top row s when it leaves the top
 //                   block, else -1.
 // Each thread traces one row through the interchange sequence.
-__global__ void perm_kernel(const int* ipiv, int ia, int jb, int* permU) {
+HPLB_DEV void trace_perm(const int* ipiv, int ia, int jb, int* permU) {
   extern __shared__ int s_piv[];
   for(int i = threadIdx.x; i < jb; i += blockDim.x) s_piv[i] = ipiv[i] - ia;
   __syncthreads();
@@ -841,6 +841,13 @@ __global__ void perm_kernel(const int* ipiv, int ia, int jb, int* permU) {
     }
     permU[jb + x] = pos >= jb ? pos : -1;
   }
+}
+__global__ void perm_kernel(const int* ipiv, int ia, int jb, int* permU) {
+  trace_perm(ipiv, ia, jb, permU);
+}
+__global__ void perm_panels_kernel(const int* ipiv, int n, int nb, int* permU) {
+  const int j = (int)blockIdx.x * nb;
+  trace_perm(ipiv + j, j, min(nb, n - j), permU + (size_t)2 * nb * blockIdx.x);
 }
 
 // Inverses of the unit-lower kTri x kTri diagonal blocks of L (n x n at
@@ -1314,6 +1321,12 @@ cudaError_t launch_panel_swap(T* A, int64_t ld, const int* ipiv, int r0, int c0,
 cudaError_t launch_perm(const int* ipiv, int ia, int jb, int* permU, cudaStream_t stream) {
   if(jb <= 0) return cudaSuccess;
   perm_kernel<<<1, 1024, jb * sizeof(int), stream>>>(ipiv, ia, jb, permU);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_perm_panels(const int* ipiv, int n, int nb, int* permU, cudaStream_t stream) {
+  if(n <= 0) return cudaSuccess;
+  perm_panels_kernel<<<(n + nb - 1) / nb, 1024, nb * sizeof(int), stream>>>(ipiv, n, nb, permU);
   return cudaGetLastError();
 }
 

@@ -137,60 +137,22 @@ __global__ void rows_xform_kernel(int jb, const double* __restrict__ in, int64_t
   }
 }
 
-// X (jb x ncols) <- L^-1 X for a unit-lower L and few right-hand sides: one
-// CTA per column, the column in shared memory.  Per 32-row block the 16 warps
-// split the dot products of the block's rows with the solved rows above (lane
-// = row, so each step reads 32 consecutive entries of a column of L), a fixed
-// order sum of the 16 slices, then the block's 32 x 32 inverse (dinv, from
-// diag_inv) applied.
-constexpr int kSmallThreads = 512;
-__global__ void __launch_bounds__(kSmallThreads)
-trsm_small_kernel(int jb, double* X, int64_t ldx, const double* __restrict__ L, int64_t ldl,
-                  const double* __restrict__ dinv) {
-  extern __shared__ double xs[];
-  __shared__ double part[kSmallThreads / 32][33];
-  __shared__ double tmp[32];
-  double*   col  = X + (size_t)blockIdx.x * ldx;
-  const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5, nsl = kSmallThreads / 32;
-  for(int i = threadIdx.x; i < jb; i += kSmallThreads) xs[i] = col[i];
-  __syncthreads();
-  for(int b0 = 0; b0 < jb; b0 += 32) {
-    const int r   = b0 + lane;
-    double    acc = 0.0, acc2 = 0.0;
-    if(r < jb) {
-      const double* lr = L + r;
-      int           k  = sl;
-      for(; k + 7 * nsl < b0; k += 8 * nsl) {  // eight loads in flight, two chains
-        double a[8];
-#pragma unroll
-        for(int q = 0; q < 8; ++q) a[q] = lr[(size_t)(k + q * nsl) * ldl];
-#pragma unroll
-        for(int q = 0; q < 8; q += 2) {
-          acc  = fma(a[q], xs[k + q * nsl], acc);
-          acc2 = fma(a[q + 1], xs[k + (q + 1) * nsl], acc2);
-        }
-      }
-      for(; k < b0; k += nsl) acc = fma(lr[(size_t)k * ldl], xs[k], acc);
-      acc += acc2;
-    }
-    part[sl][lane] = acc;
-    __syncthreads();
-    if(threadIdx.x < 32) {
-      double t = 0.0;
-      for(int q = 0; q < nsl; ++q) t += part[q][lane];
-      tmp[lane] = r < jb ? xs[r] - t : 0.0;
-    }
-    __syncthreads();
-    if(threadIdx.x < 32 && r < jb) {
-      const double* D = dinv + (size_t)(b0 / 32) * 1024;
-      double        x = 0.0;
-#pragma unroll 8
-      for(int c = 0; c < 32; ++c) x += D[c * 32 + lane] * tmp[c];
-      xs[r] = x;
-    }
-    __syncthreads();
+// A panel's interchanges on a column of X (a CTA per column): the new top rows
+// and the displaced old ones read before any row is written.
+__global__ void __launch_bounds__(256)
+permute_rows_kernel(double* X, int64_t ldx, int ia, int jb, const int* __restrict__ permU) {
+  extern __shared__ double rows[];  // 2 jb
+  double* col = X + (size_t)blockIdx.x * ldx + ia;
+  for(int x = threadIdx.x; x < jb; x += 256) {
+    rows[x]      = col[permU[x]];
+    rows[jb + x] = col[x];
   }
-  for(int i = threadIdx.x; i < jb; i += kSmallThreads) col[i] = xs[i];
+  __syncthreads();
+  for(int x = threadIdx.x; x < jb; x += 256) {
+    const int dst = permU[jb + x];
+    if(dst >= 0) col[dst] = rows[jb + x];
+    col[x] = rows[x];
+  }
 }
 
 // Split-k partial products for C (jb x nrhs) -= M (jb x K) Y (K x nrhs) with
@@ -369,12 +331,11 @@ cudaError_t launch_rows_xform(int jb, int n, const double* in, int64_t ldi, doub
   return cudaGetLastError();
 }
 
-cudaError_t launch_trsm_small(int jb, int ncols, double* X, int64_t ldx, const double* L,
-                              int64_t ldl, const double* dinv, cudaStream_t st) {
-  if(jb <= 0 || ncols <= 0) return cudaSuccess;
-  if(jb > 4096 || ncols > 65535) return cudaErrorInvalidValue;
-  trsm_small_kernel<<<ncols, kSmallThreads, (size_t)jb * sizeof(double), st>>>(jb, X, ldx, L, ldl,
-                                                                              dinv);
+cudaError_t launch_permute_rows(double* X, int64_t ldx, int ia, int jb, const int* permU, int n,
+                                cudaStream_t st) {
+  if(jb <= 0 || n <= 0) return cudaSuccess;
+  if(jb > 2048 || n > 65535) return cudaErrorInvalidValue;
+  permute_rows_kernel<<<n, 256, 2 * (size_t)jb * sizeof(double), st>>>(X, ldx, ia, jb, permU);
   return cudaGetLastError();
 }
 

@@ -10,10 +10,13 @@
 //   A^-1 = U^-1 E_{np-1} P_{np-1} ... E_0 P_0,  E_p = [L11^-1 0; -L21 L11^-1 I]
 // and
 //   A^-T = P_0^T E_0^T ... P_{np-1}^T E_{np-1}^T U^-T.
-// The off-diagonal block products are DMMA GEMMs of this library; the
-// diagonal blocks are solved by the blocked substitution kernel (explicit
-// inverses of 512 x 512 blocks would cost far more than a few right-hand
-// sides); the transposed solve reads a transposed copy of the factors so that
+// Up to 128 right-hand sides a panel's L11 and the rows below it take one
+// persistent launch per 32 of them (launch_trsm_lower): with a CTA per column for
+// L11 and a product kernel for the rows below, the chain of launches bounded the
+// solve (N = 8192, NB = 512, 32 right-hand sides: 4.25 ms, now 1.69).  More
+// right-hand sides take the blocked substitution and DMMA GEMMs (explicit
+// inverses of 512 x 512 blocks would cost far more).  The row maps of all panels
+// come from one launch; the transposed solve reads a transposed copy of the factors so that
 // its GEMMs are plain NN.
 #include <algorithm>
 
@@ -55,38 +58,38 @@ struct Rhs {
     if(nrhs <= 128) return launch_rows_sub(m, nrhs, k, M, ldm, Y, ldy, C, ldc, st);
     return launch_dgemm_sub(m, nrhs, k, M, ldm, Y, ldy, C, ldc, ctx->d_status, st);
   }
-  // Few right-hand sides: one CTA per column; many: the blocked kernel.
-  cudaError_t trsm(double* X, int64_t ldx, int jb, const double* L, int64_t ldl) {
-    if(nrhs <= 128) return launch_trsm_small(jb, nrhs, X, ldx, L, ldl, dinv, st);
-    return launch_trsm_unit_lower(X, ldx, jb, L, ldl, dinv, nrhs, st);
+  // X <- L^-1 X, L unit-lower jb x jb.  Few right-hand sides: the persistent
+  // block solve; many: the blocked substitution with 32 x 32 inverses.
+  hplb_status trsm(double* X, int64_t ldx, int jb, const double* L, int64_t ldl) {
+    hplb_ctx* ctx = this->ctx;
+    if(nrhs <= 128) {
+      CK(launch_trsm_lower(L, ldl, jb, jb, nrhs, X, ldx, ctx->d_trsv, ctx->d_status, st,
+                           &ctx->launches));
+      return HPLB_OK;
+    }
+    CK(launch_diag_inv<double>(L, ldl, 0, 0, jb, dinv, st));
+    CK(launch_trsm_unit_lower(X, ldx, jb, L, ldl, dinv, nrhs, st));
+    ctx->launches += 2;
+    return HPLB_OK;
   }
 
   const double* lu(int i, int j) const { return LU + (size_t)i + (size_t)j * (size_t)ld; }
   double*       b(int i) const { return B + i; }
+  const int*    panel_perm(int j) const { return perm + (size_t)2 * nb * (j / nb); }
   const double* t(int i, int j) const { return T + (size_t)i + (size_t)j * (size_t)ldt; }
 
-  // B[j : j + jb] <- L11^-1 B[j : j + jb], the unit-lower diagonal block of
-  // panel j, by the blocked substitution (32 x 32 diagonal inverses, then
-  // updates of the rows below), in place.
-  hplb_status solve_lower(int j, int jb) {
-    hplb_ctx* ctx = this->ctx;
-    CK(launch_diag_inv<double>(LU, ld, j, j, jb, dinv, st));
-    CK(trsm(b(j), ldb, jb, lu(j, j), ld));
-    ctx->launches += 2;
-    return HPLB_OK;
-  }
   // B[j : j + jb] <- S^-1 B[j : j + jb] for S = U11 (kind 0), L11^T (kind 1)
   // or U11^T (kind 2), each solved as the unit-lower system it is equivalent
   // to (launch_unit_lower_view): U x = b is (J D^-1 U J)(J x) = J D^-1 b,
   // L^T x = b is (J L^T J)(J x) = J b, U^T x = b is (D^-1 U)^T (D x) = b.
   hplb_status solve_view(int kind, int j, int jb) {
-    hplb_ctx* ctx = this->ctx;
+    hplb_ctx*   ctx = this->ctx;
+    hplb_status s;
     CK(launch_unit_lower_view(kind, jb, lu(j, j), ld, M1, dvec, st));
-    CK(launch_diag_inv<double>(M1, jb, 0, 0, jb, dinv, st));
     CK(launch_rows_xform(jb, nrhs, b(j), ldb, W, jb, dvec, kind != 2, kind == 0, st));
-    CK(trsm(W, jb, jb, M1, jb));
+    if((s = trsm(W, jb, jb, M1, jb)) != HPLB_OK) return s;
     CK(launch_rows_xform(jb, nrhs, W, jb, b(j), ldb, dvec, kind != 2, kind == 2, st));
-    ctx->launches += 5;
+    ctx->launches += 3;
     return HPLB_OK;
   }
 
@@ -96,13 +99,16 @@ struct Rhs {
     hplb_status s;
     for(int j = 0; j < n; j += nb) {
       const int jb = std::min(nb, n - j);
-      CK(launch_perm(ipiv + j, j, jb, perm, st));
-      CK(launch_laswp_gather<double>(B, ldb, j, jb, perm, W, jb, 0, nrhs, st));
-      CK(cudaMemcpy2DAsync(b(j), (size_t)ldb * sizeof(double), W, (size_t)jb * sizeof(double),
-                           (size_t)jb * sizeof(double), nrhs, cudaMemcpyDeviceToDevice, st));
-      if((s = solve_lower(j, jb)) != HPLB_OK) return s;
+      CK(launch_permute_rows(B, ldb, j, jb, panel_perm(j), nrhs, st));
+      ctx->launches += 1;
+      if(nrhs <= 128) {  // L11^-1 and the rows below in one launch per 32 right-hand sides
+        CK(launch_trsm_lower(lu(j, j), ld, jb, n - j, nrhs, b(j), ldb, ctx->d_trsv, ctx->d_status,
+                             st, &ctx->launches));
+        continue;
+      }
+      if((s = trsm(b(j), ldb, jb, lu(j, j), ld)) != HPLB_OK) return s;
       CK(update(n - j - jb, jb, lu(j + jb, j), ld, b(j), ldb, b(j + jb), ldb));
-      ctx->launches += 3;
+      ctx->launches += 1;
     }
     if(nrhs <= 128) {  // U X = Y in one persistent launch per 32 right-hand sides
       CK(launch_trsm_upper(LU, ld, n, nrhs, B, ldb, B, ldb, ctx->d_trsv, ctx->d_status, st,
@@ -144,9 +150,8 @@ struct Rhs {
         ctx->launches += 1;
       }
       if((s = solve_view(1, j, jb)) != HPLB_OK) return s;
-      CK(launch_perm(ipiv + j, j, jb, perm, st));
-      CK(launch_laswp_inverse(B, ldb, j, jb, perm, nrhs, st));
-      ctx->launches += 2;
+      CK(launch_laswp_inverse(B, ldb, j, jb, panel_perm(j), nrhs, st));
+      ctx->launches += 1;
     }
     return HPLB_OK;
   }
@@ -183,7 +188,8 @@ hplb_status hplb_getrs(hplb_ctx* ctx, int trans, int n, int nb, int nrhs, const 
   R.ldt  = ((int64_t)n + 15) / 16 * 16 + 16;
   hplb_status s;
   if((s = grow(ctx, &ctx->r_ws, &ctx->r_ws_cap, Rhs::ws_doubles(n, R.nb, nrhs))) != HPLB_OK ||
-     (s = grow(ctx, &ctx->r_perm, &ctx->r_perm_cap, 2 * (size_t)R.nb)) != HPLB_OK)
+     (s = grow(ctx, &ctx->r_perm, &ctx->r_perm_cap,
+               2 * (size_t)R.nb * ((n + R.nb - 1) / R.nb))) != HPLB_OK)
     return s;
   if(trans && (s = grow(ctx, &ctx->r_t, &ctx->r_t_cap, (size_t)R.ldt * n)) != HPLB_OK) return s;
   if((s = grow(ctx, &ctx->d_trsv, &ctx->trsv_cap, trsv_flag_ints(n))) != HPLB_OK) return s;
@@ -203,6 +209,8 @@ hplb_status hplb_getrs(hplb_ctx* ctx, int trans, int n, int nb, int nrhs, const 
   ctx->launches = 0;
   cudaEvent_t e0 = next_event(ctx), e1 = next_event(ctx);
   CK(cudaEventRecord(e0, R.st));
+  CK(launch_perm_panels(d_ipiv, n, R.nb, R.perm, R.st));
+  ctx->launches += 1;
   if((s = trans ? R.solve_t() : R.solve()) != HPLB_OK) return s;
   CK(cudaEventRecord(e1, R.st));
   {

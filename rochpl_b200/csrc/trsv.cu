@@ -85,7 +85,8 @@ HPLB_DEV void load_tile(const double* __restrict__ A, int64_t ld, int r0, int c0
 // In-place inverse of the upper triangular kTb x kTb block T (column by
 // column, left to right: column j of the inverse is -T_jj^-1 times the
 // already-inverted leading block applied to column j of U).  256 threads.
-HPLB_DEV void invert_upper(double (*T)[kTb + 1]) {
+template <int PITCH>
+HPLB_DEV void invert_upper(double (*T)[PITCH]) {
   const int t = threadIdx.x, row = t >> 2, part = t & 3;
   for(int j = 0; j < kTb; ++j) {
     double s = 0.0;
@@ -178,27 +179,35 @@ trsv_kernel(const double* __restrict__ A, int64_t ld, int n, const double* __res
   if(t == 0) st_release_gpu(flags + bi, 1);
 }
 
-// ---- U X = Y for up to kNr right-hand sides per launch ----
+// ---- triangular solves with up to kNr right-hand sides per launch ----
 //
-// trsv_kernel's structure with a kTb x kNr block of unknowns per row block:
-// CTA k (ticket order) owns row block bi = nblk - 1 - k and walks its row
-// panel bottom-up.  Each 64 x 64 tile of U is staged in shared memory by
-// asynchronous copies (two buffers: the next tile lands while the current one
-// is used) beside the published block x_j, and every warp accumulates
-// U[bi, j] x_j for its own kNr / 8 right-hand sides (lane = rows 2 lane and
-// 2 lane + 1), so each element of U crosses HBM once and feeds kNr FMAs.
-// Then x_bi = U_ii^-1 (y_bi - sum), with U_ii inverted while the first tile
-// loads.  Waits are bounded (status site 42).  X may alias Y: block bi of Y is
-// read only by its own CTA, before that CTA writes block bi of X.
-constexpr int kNr        = 32;                // right-hand sides per launch
-constexpr int kNrPerWarp = kNr / kTrsvWarps;  // 4
-constexpr int kTrsmSite  = 42;
+// trsv_kernel's structure for blocks of kTb rows x kNg right-hand sides.  Upper:
+// U X = Y from the last row block up.  Lower: X <- L^-1 X for the unit-lower
+// ns x ns L from the first row block down, and for the rows below it (up to
+// rows) X -= L21 X_top, their tiles consumed as the blocks of X_top appear.  A
+// CTA (ticket order: it waits only for CTAs that started before it) owns one row
+// block of one group of right-hand sides and walks its row panel; each 64 x 64
+// tile is staged by asynchronous copies (two buffers) beside the published block
+// x_j, and the CTA's product is a DMMA m16n8k8 per warp and 8 columns (4 row
+// tiles, the 64 columns in two halves).  Then x = D^-1 (y - sum) with the
+// diagonal block inverted while the first tile lands.
+//
+// Bound by the chain of row blocks: flag, x_j, one tile product, D^-1 product,
+// store, flag.  Eight right-hand sides per CTA (four CTAs share a tile through
+// L2) and the tensor-core products keep that chain short: the earlier form, 32
+// right-hand sides per CTA with FMA loops bound by shared-memory loads, took
+// 12.3 us per row block (N = 8192: 1576 us, now 424 us).  Waits are bounded
+// (status site 42).  X may alias Y: a block of Y is read only by its own CTA,
+// before that CTA writes X there.
+constexpr int kNr       = 32;       // right-hand sides per launch
+constexpr int kNg       = 8;        // right-hand sides per CTA
+constexpr int kTp       = kTb + 4;  // pitch = 4 mod 16: fragment loads free of conflicts
+constexpr int kTrsmSite = 42;
 
 struct TrsmSmem {
-  double U[2][kTb][kTb];      // staged tiles, [column][row]
-  double X[2][kTb][kNr + 2];  // the staged tile's x_j, [row of block j][rhs]
-  double T[kTb][kTb + 1];     // U_ii, then U_ii^-1
-  double R[kTb][kNr + 1];     // y_bi - sum_j U_ij x_j, [row][rhs]
+  double U[2][kTb][kTp];  // staged tiles, [column][row]
+  double X[2][kNg][kTp];  // the staged tile's x_j, [rhs][row]; then y - sum
+  double T[kTb][kTp];     // the diagonal block (lower: transposed), then its inverse
   int    ticket;
 };
 
@@ -214,12 +223,19 @@ HPLB_DEV void cp_async8(void* dst, const void* src, int bytes) {
                "l"(src), "r"(bytes)
                : "memory");
 }
+HPLB_DEV void dmma(double (&d)[4], const double (&a)[4], const double (&b)[2]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 "
+      "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
 
 // Copies of the tile rows r0 .. r0 + kb, columns c0 .. c0 + kc of A into U
 // (zeros outside), as one commit group.  VEC: 16-byte copies of row pairs (A
-// 16-byte aligned, ld even); else 8-byte copies.
+// 16-byte aligned, ld and r0 even); else 8-byte copies.
 template <bool VEC>
-HPLB_DEV void stage_tile(double (*U)[kTb], const double* A, int64_t ld, int r0, int kb, int c0,
+HPLB_DEV void stage_tile(double (*U)[kTp], const double* A, int64_t ld, int r0, int kb, int c0,
                          int kc) {
   if(VEC) {
     for(int id = threadIdx.x; id < kTb * kTb / 2; id += kTrsvThreads) {
@@ -239,96 +255,136 @@ HPLB_DEV void stage_tile(double (*U)[kTb], const double* A, int64_t ld, int r0, 
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
-template <bool VEC>
-__global__ void __launch_bounds__(kTrsvThreads, 1)
-trsm_upper_kernel(const double* __restrict__ A, int64_t ld, int n, int nrhs, const double* Y,
-                  int64_t ldy, double* X, int64_t ldx, int* flags, int* status) {
+template <bool LOWER, bool VEC>
+__global__ void __launch_bounds__(kTrsvThreads, 2)
+trsm_kernel(const double* __restrict__ A, int64_t ld, int ns, int rows, int nrhs, const double* Y,
+            int64_t ldy, double* X, int64_t ldx, int* flags, int* status) {
   extern __shared__ __align__(16) unsigned char trsm_smem_raw[];
   TrsmSmem& S    = *reinterpret_cast<TrsmSmem*>(trsm_smem_raw);
-  const int nblk = (n + kTb - 1) / kTb;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  if(t == 0) S.ticket = atomicAdd(flags + nblk, 1);
+  const int nblk = (ns + kTb - 1) / kTb, ng = (nrhs + kNg - 1) / kNg;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, g = lane >> 2, t4 = lane & 3;
+  if(t == 0) S.ticket = atomicAdd(flags + nblk * ng, 1);
   __syncthreads();
-  const int bi = nblk - 1 - S.ticket;
-  const int r0 = bi * kTb;
-  const int kb = min(kTb, n - r0);
-  const int q0 = warp * kNrPerWarp;  // this warp's right-hand sides
+  const int  grp = S.ticket % ng, blk = S.ticket / ng;
+  const bool solve = blk < nblk;  // false: rows below the lower triangle
+  const int  bi = LOWER ? blk : nblk - 1 - blk;
+  const int  r0 = solve ? bi * kTb : ns + (blk - nblk) * kTb;
+  const int  kb = min(kTb, (solve ? ns : rows) - r0);
+  const int  nt = min(blk, nblk);  // tiles of the row panel
+  const int  q0 = grp * kNg, nq = min(kNg, nrhs - q0);
+  const int  rt = (warp & 3) * 16, kh = (warp >> 2) * (kTb / 2);
+  auto       tile = [&](int i) { return LOWER ? i : nblk - 1 - i; };
+  if(nt > 0) stage_tile<VEC>(S.U[0], A, ld, r0, kb, tile(0) * kTb, min(kTb, ns - tile(0) * kTb));
 
-  int j = nblk - 1;
-  if(j > bi) stage_tile<VEC>(S.U[j & 1], A, ld, r0, kb, j * kTb, min(kTb, n - j * kTb));
-
-  // Diagonal block (identity beyond kb), inverted while the first tile lands.
-  for(int idx = t; idx < kTb * kTb; idx += kTrsvThreads) {
-    const int c = idx / kTb, r = idx % kTb;
-    double    v = (r == c) ? 1.0 : 0.0;
-    if(r < kb && c < kb) v = r <= c ? A[(size_t)(r0 + r) + (size_t)(r0 + c) * (size_t)ld] : 0.0;
-    S.T[r][c] = v;
-  }
-  __syncthreads();
-  invert_upper(S.T);
-
-  double acc[2][kNrPerWarp];
-#pragma unroll
-  for(int h = 0; h < 2; ++h)
-#pragma unroll
-    for(int k = 0; k < kNrPerWarp; ++k) acc[h][k] = 0.0;
-  bool alive = true;
-  for(; j > bi; --j) {
-    const int b  = j & 1;
-    const int kc = min(kTb, n - j * kTb);
-    if(alive) alive = wait_flag(flags + j, status, kTrsmSite);
-    for(int id = t; id < kTb * kNr; id += kTrsvThreads) {
-      const int r = id % kTb, q = id / kTb;
-      S.X[b][r][q] =
-          (r < kc && q < nrhs) ? __ldcg(X + (size_t)(j * kTb + r) + (size_t)q * (size_t)ldx) : 0.0;
+  if(solve) {  // the diagonal block (identity beyond kb), inverted
+    for(int idx = t; idx < kTb * kTb; idx += kTrsvThreads) {
+      const int c = idx / kTb, r = idx % kTb;
+      double    v = (r == c) ? 1.0 : 0.0;
+      if(r < kb && c < kb) {
+        if(LOWER)
+          v = r > c ? A[(size_t)(r0 + r) + (size_t)(r0 + c) * (size_t)ld] : v;
+        else
+          v = r <= c ? A[(size_t)(r0 + r) + (size_t)(r0 + c) * (size_t)ld] : 0.0;
+      }
+      if(LOWER)
+        S.T[c][r] = v;
+      else
+        S.T[r][c] = v;
     }
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");  // this thread's copies of tile j
+    __syncthreads();
+    invert_upper(S.T);
+  }
+  double y[4];  // this warp's entries of y (the warps of the first half)
+#pragma unroll
+  for(int e = 0; e < 4; ++e) {
+    const int r = rt + g + (e >> 1) * 8, q = 2 * t4 + (e & 1);
+    y[e] = (kh == 0 && r < kb && q < nq) ? Y[(size_t)(r0 + r) + (size_t)(q0 + q) * (size_t)ldy]
+                                         : 0.0;
+  }
+
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  bool   alive  = true;
+  for(int i = 0; i < nt; ++i) {
+    const int b = i & 1, j = tile(i), kc = min(kTb, ns - j * kTb);
+    if(alive) alive = wait_flag(flags + j * ng + grp, status, kTrsmSite);
+#pragma unroll
+    for(int h = 0; h < kTb * kNg / kTrsvThreads; ++h) {
+      const int r = t % kTb, q = t / kTb + h * (kTrsvThreads / kTb);
+      S.X[b][q][r] = (r < kc && q < nq)
+                         ? __ldcg(X + (size_t)(j * kTb + r) + (size_t)(q0 + q) * (size_t)ldx)
+                         : 0.0;
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");  // this thread's copies of the tile
     __syncthreads();  // everyone's, and the other buffers are no longer read
-    if(j - 1 > bi) stage_tile<VEC>(S.U[b ^ 1], A, ld, r0, kb, (j - 1) * kTb, kTb);
-#pragma unroll 4
-    for(int c = 0; c < kTb; ++c) {
-      const double2 u   = *reinterpret_cast<const double2*>(&S.U[b][c][2 * lane]);
-      const double2 x01 = *reinterpret_cast<const double2*>(&S.X[b][c][q0]);
-      const double2 x23 = *reinterpret_cast<const double2*>(&S.X[b][c][q0 + 2]);
-      acc[0][0] = fma(u.x, x01.x, acc[0][0]);
-      acc[0][1] = fma(u.x, x01.y, acc[0][1]);
-      acc[0][2] = fma(u.x, x23.x, acc[0][2]);
-      acc[0][3] = fma(u.x, x23.y, acc[0][3]);
-      acc[1][0] = fma(u.y, x01.x, acc[1][0]);
-      acc[1][1] = fma(u.y, x01.y, acc[1][1]);
-      acc[1][2] = fma(u.y, x23.x, acc[1][2]);
-      acc[1][3] = fma(u.y, x23.y, acc[1][3]);
+    if(i + 1 < nt)
+      stage_tile<VEC>(S.U[b ^ 1], A, ld, r0, kb, tile(i + 1) * kTb,
+                      min(kTb, ns - tile(i + 1) * kTb));
+#pragma unroll
+    for(int s = 0; s < kTb / 2; s += 8) {
+      const int    k    = kh + s + t4;
+      const double a[4] = {S.U[b][k][rt + g], S.U[b][k][rt + g + 8], S.U[b][k + 4][rt + g],
+                           S.U[b][k + 4][rt + g + 8]};
+      const double x[2] = {S.X[b][g][k], S.X[b][g][k + 4]};
+      dmma(acc, a, x);
     }
   }
 
-  // R = y_bi - sum, then x_bi = U_ii^-1 R (lane = rows lane and lane + 32).
-#pragma unroll
-  for(int h = 0; h < 2; ++h)
-#pragma unroll
-    for(int k = 0; k < kNrPerWarp; ++k) {
-      const int    r = 2 * lane + h, q = q0 + k;
-      const double y = (r < kb && q < nrhs) ? Y[(size_t)(r0 + r) + (size_t)q * (size_t)ldy] : 0.0;
-      S.R[r][q]      = y - acc[h][k];
-    }
+  // y - sum: the second half's part through shared memory.
   __syncthreads();
+  if(kh != 0)
 #pragma unroll
-  for(int h = 0; h < 2; ++h) {
-    const int r = lane + 32 * h;
-    double    x[kNrPerWarp];
+    for(int e = 0; e < 4; ++e) S.X[1][2 * t4 + (e & 1)][rt + g + (e >> 1) * 8] = acc[e];
+  __syncthreads();
+  if(kh == 0) {
 #pragma unroll
-    for(int k = 0; k < kNrPerWarp; ++k) x[k] = 0.0;
-    for(int m = r; m < kTb; ++m) {
-      const double tv = S.T[r][m];
-#pragma unroll
-      for(int k = 0; k < kNrPerWarp; ++k) x[k] = fma(tv, S.R[m][q0 + k], x[k]);
+    for(int e = 0; e < 4; ++e) {
+      const int r = rt + g + (e >> 1) * 8, q = 2 * t4 + (e & 1);
+      y[e] -= acc[e] + S.X[1][q][r];
+      S.X[0][q][r] = y[e];
     }
-#pragma unroll
-    for(int k = 0; k < kNrPerWarp; ++k)
-      if(r < kb && q0 + k < nrhs) X[(size_t)(r0 + r) + (size_t)(q0 + k) * (size_t)ldx] = x[k];
   }
-  __threadfence();
+  if(!solve) {
+    if(kh == 0)
+#pragma unroll
+      for(int e = 0; e < 4; ++e) {
+        const int r = rt + g + (e >> 1) * 8, q = 2 * t4 + (e & 1);
+        if(r < kb && q < nq) X[(size_t)(r0 + r) + (size_t)(q0 + q) * (size_t)ldx] = y[e];
+      }
+    return;
+  }
   __syncthreads();
-  if(t == 0) st_release_gpu(flags + bi, 1);
+  if(kh == 0) {  // x = D^-1 (y - sum), two chains
+    double x0[4] = {0.0, 0.0, 0.0, 0.0}, x1[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for(int s = 0; s < kTb; s += 8) {
+      const int k = s + t4, r = rt + g;
+      double    a[4];
+      if(LOWER) {
+        a[0] = S.T[k][r];
+        a[1] = S.T[k][r + 8];
+        a[2] = S.T[k + 4][r];
+        a[3] = S.T[k + 4][r + 8];
+      } else {
+        a[0] = S.T[r][k];
+        a[1] = S.T[r + 8][k];
+        a[2] = S.T[r][k + 4];
+        a[3] = S.T[r + 8][k + 4];
+      }
+      const double v[2] = {S.X[0][g][k], S.X[0][g][k + 4]};
+      if(s & 8)
+        dmma(x1, a, v);
+      else
+        dmma(x0, a, v);
+    }
+#pragma unroll
+    for(int e = 0; e < 4; ++e) {
+      const int r = rt + g + (e >> 1) * 8, q = 2 * t4 + (e & 1);
+      if(r < kb && q < nq) X[(size_t)(r0 + r) + (size_t)(q0 + q) * (size_t)ldx] = x0[e] + x1[e];
+    }
+    __threadfence();
+  }
+  __syncthreads();
+  if(t == 0) st_release_gpu(flags + bi * ng + grp, 1);
 }
 
 // z[r] += sum_c U[r, c] x[c] for r < m, c < k: a thread per row (coalesced
@@ -361,7 +417,7 @@ __global__ void vsub_kernel(int n, const double* __restrict__ y, const double* _
 
 }  // namespace
 
-size_t trsv_flag_ints(int n) { return (size_t)(n + kTb - 1) / kTb + 1; }
+size_t trsv_flag_ints(int n) { return (size_t)(n + kTb - 1) / kTb * (kNr / kNg) + 1; }
 
 cudaError_t launch_gemv_acc(int m, int k, const double* U, int64_t ld, const double* x,
                             double* z, cudaStream_t stream) {
@@ -396,41 +452,63 @@ cudaError_t launch_trsv_y(const double* A, int64_t ld, int n, const double* Y, d
   return cudaGetLastError();
 }
 
-cudaError_t launch_trsm_upper(const double* A, int64_t ld, int n, int nrhs, const double* Y,
-                              int64_t ldy, double* X, int64_t ldx, int* flags, int* status,
-                              cudaStream_t stream, int* launches) {
-  if(n <= 0 || nrhs <= 0) return cudaSuccess;
-  const int  nblk = (n + kTb - 1) / kTb;
-  const bool vec  = (reinterpret_cast<uintptr_t>(A) % 16 == 0) && (ld % 2 == 0);
+namespace {
+
+template <bool LOWER, bool VEC>
+cudaError_t launch_trsm_form(const double* A, int64_t ld, int ns, int rows, int nrhs,
+                             const double* Y, int64_t ldy, double* X, int64_t ldx, int* flags,
+                             int* status, cudaStream_t stream) {
   static bool attr = false;
   if(!attr) {
-    cudaError_t e = cudaFuncSetAttribute(trsm_upper_kernel<true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)sizeof(TrsmSmem));
-    if(e == cudaSuccess)
-      e = cudaFuncSetAttribute(trsm_upper_kernel<false>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrsmSmem));
+    const cudaError_t e = cudaFuncSetAttribute(
+        trsm_kernel<LOWER, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrsmSmem));
     if(e != cudaSuccess) return e;
     attr = true;
   }
-  // One launch per group of kNr right-hand sides, each with fresh flags.
+  const int blocks = (ns + kTb - 1) / kTb + (rows - ns + kTb - 1) / kTb;
+  trsm_kernel<LOWER, VEC><<<blocks * ((nrhs + kNg - 1) / kNg), kTrsvThreads, sizeof(TrsmSmem),
+                            stream>>>(A, ld, ns, rows, nrhs, Y, ldy, X, ldx, flags, status);
+  return cudaGetLastError();
+}
+
+// One launch per group of kNr right-hand sides, each with fresh flags.
+template <bool LOWER>
+cudaError_t launch_trsm_blocks(const double* A, int64_t ld, int ns, int rows, int nrhs,
+                               const double* Y, int64_t ldy, double* X, int64_t ldx, int* flags,
+                               int* status, cudaStream_t stream, int* launches) {
+  if(ns <= 0 || nrhs <= 0) return cudaSuccess;
+  const bool vec = reinterpret_cast<uintptr_t>(A) % 16 == 0 && ld % 2 == 0 &&
+                   (rows == ns || ns % 2 == 0);
   for(int q = 0; q < nrhs; q += kNr) {
     const int   nr = std::min(kNr, nrhs - q);
-    cudaError_t e  = cudaMemsetAsync(flags, 0, trsv_flag_ints(n) * sizeof(int), stream);
+    cudaError_t e  = cudaMemsetAsync(flags, 0, trsv_flag_ints(ns) * sizeof(int), stream);
     if(e != cudaSuccess) return e;
     const double* Yq = Y + (size_t)q * (size_t)ldy;
     double*       Xq = X + (size_t)q * (size_t)ldx;
-    if(vec)
-      trsm_upper_kernel<true><<<nblk, kTrsvThreads, sizeof(TrsmSmem), stream>>>(
-          A, ld, n, nr, Yq, ldy, Xq, ldx, flags, status);
-    else
-      trsm_upper_kernel<false><<<nblk, kTrsvThreads, sizeof(TrsmSmem), stream>>>(
-          A, ld, n, nr, Yq, ldy, Xq, ldx, flags, status);
-    ++*launches;
-    e = cudaGetLastError();
+    e = vec ? launch_trsm_form<LOWER, true>(A, ld, ns, rows, nr, Yq, ldy, Xq, ldx, flags, status,
+                                            stream)
+            : launch_trsm_form<LOWER, false>(A, ld, ns, rows, nr, Yq, ldy, Xq, ldx, flags, status,
+                                             stream);
     if(e != cudaSuccess) return e;
+    ++*launches;
   }
   return cudaSuccess;
+}
+
+}  // namespace
+
+cudaError_t launch_trsm_upper(const double* A, int64_t ld, int n, int nrhs, const double* Y,
+                              int64_t ldy, double* X, int64_t ldx, int* flags, int* status,
+                              cudaStream_t stream, int* launches) {
+  return launch_trsm_blocks<false>(A, ld, n, n, nrhs, Y, ldy, X, ldx, flags, status, stream,
+                                   launches);
+}
+
+cudaError_t launch_trsm_lower(const double* L, int64_t ldl, int ns, int rows, int nrhs, double* X,
+                              int64_t ldx, int* flags, int* status, cudaStream_t stream,
+                              int* launches) {
+  return launch_trsm_blocks<true>(L, ldl, ns, rows, nrhs, X, ldx, X, ldx, flags, status, stream,
+                                  launches);
 }
 
 }  // namespace hplb
