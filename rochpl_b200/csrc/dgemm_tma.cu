@@ -24,7 +24,9 @@
 // sets have distinct (bit0, bit3) -- what the B swizzle needs -- and distinct
 // (bit1, bit2) -- what the A swizzle needs -- so both fragments load without
 // bank conflicts.
-// A CTA computes tpc consecutive 128 x 128 tiles of a grouped order (4 column
+// Products whose 128 x 128 tiles would leave SMs idle take 64 x 64 tiles (4 warps,
+// the same slice layout with half the rows and columns) instead.
+// A CTA computes tpc consecutive tiles of a grouped order (4 column
 // tiles per A row-tile), so an A tile is fetched from HBM once and re-read
 // from L2 three times.  Either CTAs retire every few tiles, so that the
 // high-priority panel stream can get onto SMs as they free up, or (a cap on
@@ -45,14 +47,24 @@ namespace hplb {
 
 namespace {
 
-constexpr int BM = 128, BN = 128, BK = 16, STAGES = 6;
-constexpr int NCONS   = 8;               // consumer warps (one of them refills each slot)
-constexpr int THREADS = NCONS * 32;
-constexpr int GROUP_N = 4;               // column tiles per group
-constexpr int A_BYTES = BM * BK * 8;     // 16 KB
-constexpr int B_BYTES = BN * BK * 8;     // 16 KB
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int SMEM_BYTES  = STAGES * STAGE_BYTES + 1024 /*align*/ + 128 /*barriers*/;
+constexpr int BK = 16, STAGES = 6;
+constexpr int GROUP_N = 4;  // column tiles per group
+// Tile of a CTA: MW x NW warps of MI x 16 rows and NJ x 8 columns each.
+template <int MW, int NW, int MI, int NJ>
+struct TileShape {
+  static constexpr int mw = MW, mi = MI, nj = NJ;
+  static constexpr int BM = MW * MI * 16, BN = NW * NJ * 8;
+  static constexpr int NCONS   = MW * NW;  // consumer warps (one of them refills each slot)
+  static constexpr int THREADS = NCONS * 32;
+  static constexpr int A_BYTES = BM * BK * 8, B_BYTES = BN * BK * 8;
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int SMEM_BYTES  = STAGES * STAGE_BYTES + 1024 /*align*/ + 128 /*barriers*/;
+};
+// The large tile: 8 warps of 64 x 32, one CTA per SM.  The small one: 4 warps of
+// 32 x 32, two CTAs per SM, for products whose large tiles leave SMs idle (the
+// rule is in launch_dgemm_tma).
+using Large = TileShape<2, 4, 4, 4>;
+using Small = TileShape<2, 2, 2, 4>;
 
 HPLB_DEV uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -133,6 +145,7 @@ HPLB_DEV int b_off(int n, int k) {
 
 // Issue the copies of k-slice q (tile t_begin + q / KT, k-slice q % KT) into
 // ring slot q % STAGES.
+template <class S>
 HPLB_DEV void issue_slice(int q, int t_begin, int KT, int tiles_m, int tiles_n,
                           const CUtensorMap* tmA, const CUtensorMap* tmB, unsigned char* sA,
                           unsigned char* sB, uint64_t* full) {
@@ -141,21 +154,21 @@ HPLB_DEV void issue_slice(int q, int t_begin, int KT, int tiles_m, int tiles_n,
   tile_coords(t_begin + q / KT, tiles_m, tiles_n, tm, tn);
   const int kt = q % KT;
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  mbar_expect_tx(&full[s], STAGE_BYTES);
-  tma_load_3d(sA + s * A_BYTES, tmA, &full[s], 0, kt * BK, tm * (BM / 16));
-  tma_load_2d(sB + s * B_BYTES, tmB, &full[s], kt * BK, tn * BN);
+  mbar_expect_tx(&full[s], S::STAGE_BYTES);
+  tma_load_3d(sA + s * S::A_BYTES, tmA, &full[s], 0, kt * BK, tm * (S::BM / 16));
+  tma_load_2d(sB + s * S::B_BYTES, tmB, &full[s], kt * BK, tn * S::BN);
 }
 
-template <bool ACCUM>
-__global__ void __launch_bounds__(THREADS, 1)
+template <class S, bool ACCUM>
+__global__ void __launch_bounds__(S::THREADS, S::THREADS == 256 ? 1 : 2)
 dgemm_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  int m, int n, int k, double* __restrict__ C, int64_t ldc, int tiles_m,
                  int tiles_n, int tpc, int* status) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* sA   = base;                      // [STAGES][A_BYTES]
-  unsigned char* sB   = base + STAGES * A_BYTES;   // [STAGES][B_BYTES]
-  uint64_t*      full = (uint64_t*)(base + STAGES * STAGE_BYTES);
+  unsigned char* sB   = base + STAGES * S::A_BYTES;   // [STAGES][B_BYTES]
+  uint64_t*      full = (uint64_t*)(base + STAGES * S::STAGE_BYTES);
   __shared__ int          s_done[STAGES];  // warps finished with the slot's slice
   __shared__ volatile int s_abort;
 
@@ -174,13 +187,14 @@ dgemm_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     s_abort = 0;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     for(int q = 0; q < STAGES && q < nslices; ++q)
-      issue_slice(q, t_begin, KT, tiles_m, tiles_n, &tmA, &tmB, sA, sB, full);
+      issue_slice<S>(q, t_begin, KT, tiles_m, tiles_n, &tmA, &tmB, sA, sB, full);
   }
   __syncthreads();
 
   const int g = lane >> 2, t4 = lane & 3;
-  const int wm = (warp & 1) * 64;   // 2 warps along M
-  const int wn = (warp >> 1) * 32;  // 4 warps along N
+  constexpr int MI = S::mi, NJ = S::nj;
+  const int wm = (warp % S::mw) * (MI * 16);
+  const int wn = (warp / S::mw) * (NJ * 8);
   // Relabelled reduction index (see the layout note at the top): this lane's
   // k for a0/b0 and for a2/b1, in MMA k-steps 0 and 1.
   int kk[2][2];
@@ -206,19 +220,19 @@ dgemm_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   for(int t = t_begin; t < t_end; ++t) {
     int tm, tn;
     tile_coords(t, tiles_m, tiles_n, tm, tn);
-    const int m0 = tm * BM + wm, n0 = tn * BN + wn;
-    // Pull this warp's 64 x 32 block of C into L2 while the tile is computed.
+    const int m0 = tm * S::BM + wm, n0 = tn * S::BN + wn;
+    // Pull this warp's block of C into L2 while the tile is computed.
     {
       const int col = n0 + lane;
       if(ACCUM && col < n)
-        for(int r = m0; r < min(m0 + 64, m); r += 16)
+        for(int r = m0; r < min(m0 + MI * 16, m); r += 16)
           asm volatile("prefetch.global.L2 [%0];" ::"l"(C + (size_t)r + (size_t)col * ldc));
     }
-    double acc[4][4][4];
+    double acc[MI][NJ][4];
 #pragma unroll
-    for(int i = 0; i < 4; ++i)
+    for(int i = 0; i < MI; ++i)
 #pragma unroll
-      for(int j = 0; j < 4; ++j)
+      for(int j = 0; j < NJ; ++j)
 #pragma unroll
         for(int r = 0; r < 4; ++r) acc[i][j][r] = 0.0;
 
@@ -228,35 +242,35 @@ dgemm_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         s_abort = 1;
         return;
       }
-      const double* a = (const double*)(sA + slot * A_BYTES);
-      const double* b = (const double*)(sB + slot * B_BYTES);
+      const double* a = (const double*)(sA + slot * S::A_BYTES);
+      const double* b = (const double*)(sB + slot * S::B_BYTES);
 #pragma unroll
       for(int st = 0; st < 2; ++st) {
-        double af[4][4], bf[4][2];
+        double af[MI][4], bf[NJ][2];
 #pragma unroll
-        for(int i = 0; i < 4; ++i) {
+        for(int i = 0; i < MI; ++i) {
           af[i][0] = a[oA[st][0][0] + i * 256];
           af[i][1] = a[oA[st][0][1] + i * 256];
           af[i][2] = a[oA[st][1][0] + i * 256];
           af[i][3] = a[oA[st][1][1] + i * 256];
         }
 #pragma unroll
-        for(int j = 0; j < 4; ++j) {
+        for(int j = 0; j < NJ; ++j) {
           bf[j][0] = b[oB[st][0] + j * 128];
           bf[j][1] = b[oB[st][1] + j * 128];
         }
 #pragma unroll
-        for(int i = 0; i < 4; ++i)
+        for(int i = 0; i < MI; ++i)
 #pragma unroll
-          for(int j = 0; j < 4; ++j) dmma(acc[i][j], af[i], bf[j]);
+          for(int j = 0; j < NJ; ++j) dmma(acc[i][j], af[i], bf[j]);
       }
       // The last warp to finish with the slot refills it with slice q + STAGES.
       __syncwarp();
       if(lane == 0) {
-        if(atomicAdd(&s_done[slot], 1) == NCONS - 1) {
+        if(atomicAdd(&s_done[slot], 1) == S::NCONS - 1) {
           s_done[slot] = 0;
           if(q + STAGES < nslices)
-            issue_slice(q + STAGES, t_begin, KT, tiles_m, tiles_n, &tmA, &tmB, sA, sB, full);
+            issue_slice<S>(q + STAGES, t_begin, KT, tiles_m, tiles_n, &tmA, &tmB, sA, sB, full);
         }
       }
       if(++slot == STAGES) {
@@ -270,12 +284,12 @@ dgemm_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // halves; all loads of a half are issued before its stores, so they are
     // in flight together instead of one dependent round trip per element.
 #pragma unroll
-    for(int h = 0; h < 2; ++h) {
-      double cv[2][4][4];
+    for(int h = 0; h < MI / 2; ++h) {
+      double cv[2][NJ][4];
 #pragma unroll
       for(int i = 0; i < 2; ++i)
 #pragma unroll
-        for(int j = 0; j < 4; ++j)
+        for(int j = 0; j < NJ; ++j)
 #pragma unroll
           for(int r = 0; r < 4; ++r) {
             const int row = m0 + (2 * h + i) * 16 + g + (r >> 1) * 8;
@@ -286,7 +300,7 @@ dgemm_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
       for(int i = 0; i < 2; ++i)
 #pragma unroll
-        for(int j = 0; j < 4; ++j)
+        for(int j = 0; j < NJ; ++j)
 #pragma unroll
           for(int r = 0; r < 4; ++r) {
             const int row = m0 + (2 * h + i) * 16 + g + (r >> 1) * 8;
@@ -316,6 +330,19 @@ bool get_encoder() {
   return true;
 }
 
+int sm_count() {
+  static const int sms = [] {
+    int dev = 0, n = 148;
+    if(cudaGetDevice(&dev) != cudaSuccess ||
+       cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+      cudaGetLastError();
+      n = 148;
+    }
+    return n;
+  }();
+  return sms;
+}
+
 // Tiles per CTA.  Four (a whole group: the A tile fetched once and re-read
 // from L2 by the group's other column tiles, one pipeline across them) for a
 // large product, at least 256 tiles per SM -- the trailing update while it is
@@ -328,40 +355,54 @@ bool get_encoder() {
 // Measured at N = 16384 (getrf, NB = 512, B200): 251 ms with four, 208 ms
 // with one, identical bits.
 int tiles_per_cta(long long ntiles) {
-  static const int sms = [] {
-    int dev = 0, n = 148;
-    if(cudaGetDevice(&dev) != cudaSuccess ||
-       cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-      cudaGetLastError();
-      n = 148;
-    }
-    return n;
-  }();
-  return ntiles >= 1024LL * sms ? 8 : (ntiles >= 256LL * sms ? 4 : 1);
+  const long long sms = sm_count();
+  return ntiles >= 1024 * sms ? 8 : (ntiles >= 256 * sms ? 4 : 1);
 }
 
-cudaError_t launch_tpc(const CUtensorMap& mA, const CUtensorMap& mB, int m, int n, int k,
-                       double* C, int64_t ldc, int tiles_m, int tiles_n, int tpc, bool accumulate,
-                       int* status, cudaStream_t stream) {
+template <class S>
+cudaError_t launch_shape(int m, int n, int k, const double* A, int64_t lda, const double* B,
+                         int64_t ldb, double* C, int64_t ldc, int* status, bool accumulate,
+                         cudaStream_t stream, long long tpc) {
+  CUtensorMap mA, mB;
+  {
+    cuuint64_t dims[3]    = {16, (cuuint64_t)k, (cuuint64_t)((m + 15) / 16)};
+    cuuint64_t strides[2] = {(cuuint64_t)lda * 8, 128};
+    cuuint32_t box[3]     = {16, BK, S::BM / 16};
+    cuuint32_t es[3]      = {1, 1, 1};
+    CUresult r = g_encode(&mA, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, (void*)A, dims, strides, box,
+                          es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if(r != CUDA_SUCCESS) return cudaErrorInvalidValue;
+  }
+  {
+    cuuint64_t dims[2]    = {(cuuint64_t)k, (cuuint64_t)n};
+    cuuint64_t strides[1] = {(cuuint64_t)ldb * 8};
+    cuuint32_t box[2]     = {BK, S::BN};
+    cuuint32_t es[2]      = {1, 1};
+    CUresult r = g_encode(&mB, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, (void*)B, dims, strides, box,
+                          es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if(r != CUDA_SUCCESS) return cudaErrorInvalidValue;
+  }
   static bool attr = false;
   if(!attr) {
-    cudaError_t e = cudaFuncSetAttribute(dgemm_tma_kernel<true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(dgemm_tma_kernel<S, true>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM_BYTES);
     if(e == cudaSuccess)
-      e = cudaFuncSetAttribute(dgemm_tma_kernel<false>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+      e = cudaFuncSetAttribute(dgemm_tma_kernel<S, false>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM_BYTES);
     if(e != cudaSuccess) return e;
     attr = true;
   }
-  const long long ntiles = (long long)tiles_m * tiles_n;
-  const long long grid   = (ntiles + tpc - 1) / tpc;
-  if(grid > 0x7fffffff) return cudaErrorInvalidValue;
+  const int       tiles_m = (m + S::BM - 1) / S::BM, tiles_n = (n + S::BN - 1) / S::BN;
+  const long long grid    = ((long long)tiles_m * tiles_n + tpc - 1) / tpc;
+  if(grid > 0x7fffffff || tpc > 0x7fffffff) return cudaErrorInvalidValue;
   if(accumulate)
-    dgemm_tma_kernel<true><<<(unsigned)grid, THREADS, SMEM_BYTES, stream>>>(
-        mA, mB, m, n, k, C, ldc, tiles_m, tiles_n, tpc, status);
+    dgemm_tma_kernel<S, true><<<(unsigned)grid, S::THREADS, S::SMEM_BYTES, stream>>>(
+        mA, mB, m, n, k, C, ldc, tiles_m, tiles_n, (int)tpc, status);
   else
-    dgemm_tma_kernel<false><<<(unsigned)grid, THREADS, SMEM_BYTES, stream>>>(
-        mA, mB, m, n, k, C, ldc, tiles_m, tiles_n, tpc, status);
+    dgemm_tma_kernel<S, false><<<(unsigned)grid, S::THREADS, S::SMEM_BYTES, stream>>>(
+        mA, mB, m, n, k, C, ldc, tiles_m, tiles_n, (int)tpc, status);
   return cudaGetLastError();
 }
 
@@ -380,34 +421,17 @@ bool dgemm_tma_eligible(int m, int n, int k, const double* A, int64_t lda, const
 cudaError_t launch_dgemm_tma(int m, int n, int k, const double* A, int64_t lda, const double* B,
                              int64_t ldb, double* C, int64_t ldc, int* status, bool accumulate,
                              cudaStream_t stream, int max_ctas) {
-  CUtensorMap mA, mB;
-  {
-    cuuint64_t dims[3]    = {16, (cuuint64_t)k, (cuuint64_t)((m + 15) / 16)};
-    cuuint64_t strides[2] = {(cuuint64_t)lda * 8, 128};
-    cuuint32_t box[3]     = {16, BK, BM / 16};
-    cuuint32_t es[3]      = {1, 1, 1};
-    CUresult r = g_encode(&mA, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, (void*)A, dims, strides, box,
-                          es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if(r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-  }
-  {
-    cuuint64_t dims[2]    = {(cuuint64_t)k, (cuuint64_t)n};
-    cuuint64_t strides[1] = {(cuuint64_t)ldb * 8};
-    cuuint32_t box[2]     = {BK, BN};
-    cuuint32_t es[2]      = {1, 1};
-    CUresult r = g_encode(&mB, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, (void*)B, dims, strides, box,
-                          es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if(r != CUDA_SUCCESS) return cudaErrorInvalidValue;
-  }
-  const int       tiles_m = (m + BM - 1) / BM, tiles_n = (n + BN - 1) / BN;
-  const long long ntiles  = (long long)tiles_m * tiles_n;
-  long long       tpc     = tiles_per_cta(ntiles);
+  const long long ntiles =
+      (long long)((m + Large::BM - 1) / Large::BM) * ((n + Large::BN - 1) / Large::BN);
+  // Small tiles where the large ones fill at most three quarters of the SMs: the
+  // product then takes one large tile's time (k = 256: 33 us) however few there
+  // are.  Above that both need as many rounds of the SMs.  Both sum every element
+  // in the same order.
+  if(ntiles * 4 <= 3LL * sm_count())
+    return launch_shape<Small>(m, n, k, A, lda, B, ldb, C, ldc, status, accumulate, stream, 1);
+  long long tpc = tiles_per_cta(ntiles);
   if(max_ctas > 0 && (ntiles + tpc - 1) / tpc > max_ctas) tpc = (ntiles + max_ctas - 1) / max_ctas;
-  if(tpc > 0x7fffffff) return cudaErrorInvalidValue;
-  return launch_tpc(mA, mB, m, n, k, C, ldc, tiles_m, tiles_n, (int)tpc, accumulate, status,
-                    stream);
+  return launch_shape<Large>(m, n, k, A, lda, B, ldb, C, ldc, status, accumulate, stream, tpc);
 }
 
 }  // namespace hplb
