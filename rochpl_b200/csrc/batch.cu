@@ -1012,7 +1012,9 @@ __global__ void __launch_bounds__(kBT, 1) batch_getrs_kernel(const Args* pa) {
     const int s = next_system(a, S);
     if(s < 0) break;
     const Sys&    y = a.sys[s];
-    const int     n = y.n, nrhs = y.nrhs, nb = y.nb;
+    // The factors are LAPACK's whatever width they were made with; a recursive
+    // plan's value is no width (and larger than the diagonal block S holds).
+    const int     n = y.n, nrhs = y.nrhs, nb = min(y.nb, kNbMax);
     const double* L = a.LU + y.a_off;
     double*       B = a.B + y.b_off;
     const int*    ip = a.ipivc + y.p_off;
