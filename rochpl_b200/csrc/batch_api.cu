@@ -17,7 +17,12 @@
 using namespace hplb;
 
 static const int kClassUpper[HPLB_BATCH_CLASSES] = {48, 96, 192, 384, 768, INT_MAX};
-static const int kDefaultNb[HPLB_BATCH_CLASSES]  = {8, 16, 16, 16, 16, 16};
+// The built-in table is what the tuner picks on B200 for 1 to 16 right-hand
+// sides (ms per batch of 296 systems, one right-hand side, width 16 -> this
+// table: n = 40 0.19 -> 0.165, 80 0.375 -> 0.331, 160 0.97 -> 0.80, 320 3.44 ->
+// 2.64, 640 18.2 -> 10.7, 1024 53 -> 28.5).
+static const int kDefaultNb[HPLB_BATCH_CLASSES]  = {32, 32, 32, HPLB_BATCH_RECURSIVE,
+                                                    HPLB_BATCH_RECURSIVE, HPLB_BATCH_RECURSIVE};
 static const int kTuneN[HPLB_BATCH_CLASSES]      = {40, 80, 160, 320, 640, 1024};
 
 static int size_class(int n) {
