@@ -39,6 +39,10 @@ struct Rhs {
   int*          perm;
   cudaStream_t  st;
 
+  // Flags of one panel's lower solves.
+  static size_t panel_flags(int nb, int nrhs) {
+    return trsv_flag_ints(nb) * (size_t)((nrhs + 31) / 32);
+  }
   static size_t ws_doubles(int n, int nb, int nrhs) {
     const size_t nblk = (size_t)nb / 32 + 1;
     return (size_t)nb * nrhs + (size_t)nb * nb + nb + nblk * 1024 + 64 +
@@ -63,7 +67,7 @@ struct Rhs {
   hplb_status trsm(double* X, int64_t ldx, int jb, const double* L, int64_t ldl) {
     hplb_ctx* ctx = this->ctx;
     if(nrhs <= 128) {
-      CK(launch_trsm_lower(L, ldl, jb, jb, nrhs, X, ldx, ctx->d_trsv, ctx->d_status, st,
+      CK(launch_trsm_lower(L, ldl, jb, jb, nrhs, X, ldx, ctx->d_trsv, ctx->d_status, false, st,
                            &ctx->launches));
       return HPLB_OK;
     }
@@ -97,13 +101,17 @@ struct Rhs {
   hplb_status solve() {
     hplb_ctx*   ctx = this->ctx;
     hplb_status s;
+    if(nrhs <= 128)  // the flags of every panel's launches at once
+      CK(cudaMemsetAsync(ctx->d_trsv, 0,
+                         panel_flags(nb, nrhs) * ((n + nb - 1) / nb) * sizeof(int), st));
     for(int j = 0; j < n; j += nb) {
       const int jb = std::min(nb, n - j);
       CK(launch_permute_rows(B, ldb, j, jb, panel_perm(j), nrhs, st));
       ctx->launches += 1;
       if(nrhs <= 128) {  // L11^-1 and the rows below in one launch per 32 right-hand sides
-        CK(launch_trsm_lower(lu(j, j), ld, jb, n - j, nrhs, b(j), ldb, ctx->d_trsv, ctx->d_status,
-                             st, &ctx->launches));
+        CK(launch_trsm_lower(lu(j, j), ld, jb, n - j, nrhs, b(j), ldb,
+                             ctx->d_trsv + panel_flags(nb, nrhs) * (size_t)(j / nb), ctx->d_status,
+                             true, st, &ctx->launches));
         continue;
       }
       if((s = trsm(b(j), ldb, jb, lu(j, j), ld)) != HPLB_OK) return s;
@@ -192,7 +200,9 @@ hplb_status hplb_getrs(hplb_ctx* ctx, int trans, int n, int nb, int nrhs, const 
                2 * (size_t)R.nb * ((n + R.nb - 1) / R.nb))) != HPLB_OK)
     return s;
   if(trans && (s = grow(ctx, &ctx->r_t, &ctx->r_t_cap, (size_t)R.ldt * n)) != HPLB_OK) return s;
-  if((s = grow(ctx, &ctx->d_trsv, &ctx->trsv_cap, trsv_flag_ints(n))) != HPLB_OK) return s;
+  const size_t flags = R.nrhs <= 128 ? Rhs::panel_flags(R.nb, nrhs) * ((n + R.nb - 1) / R.nb) : 0;
+  if((s = grow(ctx, &ctx->d_trsv, &ctx->trsv_cap, std::max(flags, trsv_flag_ints(n)))) != HPLB_OK)
+    return s;
   R.carve(ctx->r_ws);
   R.perm = ctx->r_perm;
   R.T    = ctx->r_t;

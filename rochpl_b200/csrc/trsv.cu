@@ -84,11 +84,12 @@ HPLB_DEV void load_tile(const double* __restrict__ A, int64_t ld, int r0, int c0
 
 // In-place inverse of the upper triangular kTb x kTb block T (column by
 // column, left to right: column j of the inverse is -T_jj^-1 times the
-// already-inverted leading block applied to column j of U).  256 threads.
+// already-inverted leading block applied to column j of U).  256 threads; T is
+// the identity from row and column kb on, which takes no step.
 template <int PITCH>
-HPLB_DEV void invert_upper(double (*T)[PITCH]) {
+HPLB_DEV void invert_upper(double (*T)[PITCH], int kb) {
   const int t = threadIdx.x, row = t >> 2, part = t & 3;
-  for(int j = 0; j < kTb; ++j) {
+  for(int j = 0; j < kb; ++j) {
     double s = 0.0;
     if(row < j)
       for(int k = row + part; k < j; k += 4) s = fma(T[row][k], T[k][j], s);
@@ -131,7 +132,7 @@ trsv_kernel(const double* __restrict__ A, int64_t ld, int n, const double* __res
   }
   if(t < kTb) S.r[t] = t < kb ? Y[r0 + t] : 0.0;
   __syncthreads();
-  invert_upper(S.T);
+  invert_upper(S.T, kb);
 
   // Row panel: acc = sum_j U[bi, j] x_j over the rows 2 lane, 2 lane + 1.
   double acc0 = 0.0, acc1 = 0.0;
@@ -292,7 +293,7 @@ trsm_kernel(const double* __restrict__ A, int64_t ld, int ns, int rows, int nrhs
         S.T[r][c] = v;
     }
     __syncthreads();
-    invert_upper(S.T);
+    invert_upper(S.T, kb);
   }
   double y[4];  // this warp's entries of y (the warps of the first half)
 #pragma unroll
@@ -471,17 +472,19 @@ cudaError_t launch_trsm_form(const double* A, int64_t ld, int ns, int rows, int 
   return cudaGetLastError();
 }
 
-// One launch per group of kNr right-hand sides, each with fresh flags.
+// One launch per group of kNr right-hand sides, each with flags of its own
+// (trsv_flag_ints(ns) per group), zeroed here unless the caller has done so.
 template <bool LOWER>
 cudaError_t launch_trsm_blocks(const double* A, int64_t ld, int ns, int rows, int nrhs,
                                const double* Y, int64_t ldy, double* X, int64_t ldx, int* flags,
-                               int* status, cudaStream_t stream, int* launches) {
+                               int* status, bool zeroed, cudaStream_t stream, int* launches) {
   if(ns <= 0 || nrhs <= 0) return cudaSuccess;
   const bool vec = reinterpret_cast<uintptr_t>(A) % 16 == 0 && ld % 2 == 0 &&
                    (rows == ns || ns % 2 == 0);
   for(int q = 0; q < nrhs; q += kNr) {
     const int   nr = std::min(kNr, nrhs - q);
-    cudaError_t e  = cudaMemsetAsync(flags, 0, trsv_flag_ints(ns) * sizeof(int), stream);
+    cudaError_t e  = cudaSuccess;
+    if(!zeroed) e = cudaMemsetAsync(flags, 0, trsv_flag_ints(ns) * sizeof(int), stream);
     if(e != cudaSuccess) return e;
     const double* Yq = Y + (size_t)q * (size_t)ldy;
     double*       Xq = X + (size_t)q * (size_t)ldx;
@@ -491,6 +494,7 @@ cudaError_t launch_trsm_blocks(const double* A, int64_t ld, int ns, int rows, in
                                              stream);
     if(e != cudaSuccess) return e;
     ++*launches;
+    if(zeroed) flags += trsv_flag_ints(ns);
   }
   return cudaSuccess;
 }
@@ -500,15 +504,15 @@ cudaError_t launch_trsm_blocks(const double* A, int64_t ld, int ns, int rows, in
 cudaError_t launch_trsm_upper(const double* A, int64_t ld, int n, int nrhs, const double* Y,
                               int64_t ldy, double* X, int64_t ldx, int* flags, int* status,
                               cudaStream_t stream, int* launches) {
-  return launch_trsm_blocks<false>(A, ld, n, n, nrhs, Y, ldy, X, ldx, flags, status, stream,
-                                   launches);
+  return launch_trsm_blocks<false>(A, ld, n, n, nrhs, Y, ldy, X, ldx, flags, status, false,
+                                   stream, launches);
 }
 
 cudaError_t launch_trsm_lower(const double* L, int64_t ldl, int ns, int rows, int nrhs, double* X,
-                              int64_t ldx, int* flags, int* status, cudaStream_t stream,
-                              int* launches) {
-  return launch_trsm_blocks<true>(L, ldl, ns, rows, nrhs, X, ldx, X, ldx, flags, status, stream,
-                                  launches);
+                              int64_t ldx, int* flags, int* status, bool zeroed,
+                              cudaStream_t stream, int* launches) {
+  return launch_trsm_blocks<true>(L, ldl, ns, rows, nrhs, X, ldx, X, ldx, flags, status, zeroed,
+                                  stream, launches);
 }
 
 }  // namespace hplb
