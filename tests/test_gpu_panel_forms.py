@@ -1,0 +1,185 @@
+"""Where a rule of the panel, the triangular solves, the small GEMM tiles, the
+residual pass or the generator changes form: both sides of each line and ragged
+remainders, against the launch-per-step panel, LAPACK or the oracle."""
+import numpy as np
+import pytest
+
+from gpu_util import from_dev
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -53
+
+
+def _panel(hlib, oracle, n, jb, nbmin, rfact, kind, zero_col=None):
+    import torch
+
+    from rochpl_b200.hpl import Algo
+    from rochpl_b200.lib import LEAF_AUTO
+
+    ld = oracle.default_ld(n)
+    dA = torch.empty(ld * jb, dtype=torch.float64, device="cuda")
+    hlib.matgen_block(n, n, 0, 0, n, jb, 7, dA.data_ptr(), ld)
+    if zero_col is not None:
+        dA.view(jb, ld)[zero_col].zero_()
+    piv = torch.zeros(jb, dtype=torch.int32, device="cuda")
+    try:
+        hlib.set_leaf(kind)
+        info = hlib.panel_factor(Algo(jb, nbmin, 2, 2, rfact, 1, 0).c(), n, 0, jb, dA.data_ptr(),
+                                 ld, 0, piv.data_ptr())
+    finally:
+        hlib.set_leaf(LEAF_AUTO)
+    return dA.view(jb, ld)[:, :n].clone(), piv, info
+
+
+# Rows a cluster holds with 1, 2 and 3 rows of 32 columns per thread, 4 and 6 of
+# 16, 8 of 8, and none; CTA counts below 16; leaves of every width in a panel.
+@pytest.mark.parametrize("n,jb,nbmin,rfact", [
+    (40, 40, 32, 2), (65, 64, 8, 2), (129, 96, 16, 1), (1025, 100, 32, 0), (4096, 64, 32, 2),
+    (4097, 70, 16, 2), (8192, 256, 32, 2), (8193, 33, 32, 2), (12288, 64, 32, 1),
+    (12289, 64, 32, 2), (16384, 48, 32, 2), (16385, 64, 32, 0), (24576, 32, 32, 2),
+    (24577, 72, 32, 2), (32768, 40, 16, 2), (32769, 40, 32, 2)])
+def test_panel_forms_match_the_launch_per_step_panel(hlib, oracle, n, jb, nbmin, rfact):
+    """The cluster panel against the panel of one launch per step: identical
+    pivots; identical bits where the leaves are not split (rows <= 12288), else
+    every entry within its summation error (jb products of |l| <= 1 and u)."""
+    from rochpl_b200.lib import LEAF_AUTO, LEAF_REGISTERS
+
+    a, pa, ia = _panel(hlib, oracle, n, jb, nbmin, rfact, LEAF_AUTO)
+    b, pb, ib = _panel(hlib, oracle, n, jb, nbmin, rfact, LEAF_REGISTERS)
+    assert ia == ib == 0 and pa.tolist() == pb.tolist()
+    if n <= 12288:
+        assert bool((a == b).all())
+    else:
+        umax = float(b[:, :jb].abs().max())
+        # Backward error of both orders, carried through the jb x jb unit-lower
+        # solve of a panel whose multipliers partial pivoting keeps below 1.
+        assert float((a - b).abs().max()) <= 64 * jb * jb * EPS * max(umax, 1.0)
+
+
+def test_panel_zero_pivot(hlib, oracle):
+    from rochpl_b200.lib import LEAF_AUTO
+
+    for n in (100, 5000, 13000):
+        assert _panel(hlib, oracle, n, 64, 32, 2, LEAF_AUTO, zero_col=37)[2] == 38
+
+
+@pytest.mark.parametrize("n,nb,nrhs", [(1, 1, 1), (63, 64, 7), (64, 64, 8), (65, 64, 9),
+                                       (130, 65, 33), (200, 200, 31), (257, 48, 40),
+                                       (300, 33, 128), (300, 64, 129)])
+@pytest.mark.parametrize("trans", [0, 1])
+def test_getrs_block_edges(hlib, oracle, n, nb, nrhs, trans):
+    import torch
+
+    from rochpl_b200.hpl import Algo
+
+    M = oracle.matgen(n, n + nrhs, 11)
+    A, B = np.array(M[:n, :n]), np.array(M[:n, n:])
+    LU = torch.from_numpy(np.ascontiguousarray(A.T)).cuda()
+    X = torch.from_numpy(np.ascontiguousarray(B.T)).cuda()
+    piv = torch.zeros(n, dtype=torch.int32, device="cuda")
+    nbe = min(nb, n)
+    assert hlib.getrf(Algo(nbe, min(16, nbe), 2, 2, 2, 1, 0).c(), n, LU.data_ptr(), n,
+                      piv.data_ptr()) == 0
+    hlib.getrs(trans, n, nbe, nrhs, LU.data_ptr(), n, piv.data_ptr(), X.data_ptr(), n)
+    ref = np.linalg.solve(A.T if trans else A, B)
+    tol = 64 * n * EPS * np.linalg.cond(A, np.inf)
+    err = np.max(np.abs(X.cpu().numpy().T - ref)) / np.max(np.abs(ref))
+    assert err <= tol, (err, tol)
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, 512, 2047, 2049])
+def test_residual_pass_edges(hlib, oracle, n):
+    """One read of the stored matrix: the regenerated check's bits, the oracle's
+    norms."""
+    import torch
+
+    ld = oracle.default_ld(n)
+    dA = torch.empty(ld * (n + 1), dtype=torch.float64, device="cuda")
+    hlib.matgen(n, n + 1, 100, dA.data_ptr(), ld)
+    x = (np.arange(n) % 7 - 3.0) / 5
+    dX = torch.from_numpy(x).cuda()
+    d1 = hlib.residual(n, dA.data_ptr(), ld, dX.data_ptr())
+    d2 = hlib.residual_lcg(n, 100, dX.data_ptr())
+    o = oracle.residual(oracle.matgen(n, n + 1, 100, ld=ld), n, x)
+    assert d1 == d2
+    for k in ("rnorm_inf", "anorm_1", "anorm_inf", "xnorm_1", "bnorm_inf"):
+        assert d1[k] == pytest.approx(o[k], rel=4 * n * EPS, abs=1e-300), k
+
+
+def test_matgen_long_runs(hlib, oracle):
+    """Tall matrices take 64-row runs; the last run of a column is ragged."""
+    import torch
+
+    m, n = 5001, 3400
+    ld = oracle.default_ld(m)
+    dA = torch.full((ld * n,), np.nan, dtype=torch.float64, device="cuda")
+    hlib.matgen(m, n, 3, dA.data_ptr(), ld)
+    got = from_dev(dA, ld, n)
+    assert np.array_equal(got[:m].view(np.uint64), oracle.matgen(m, n, 3, ld=ld)[:m].view(np.uint64))
+    assert np.all(np.isnan(got[m:]))
+
+
+@pytest.mark.parametrize("m,n,k", [(1400, 1250, 40), (1408, 1536, 96), (129, 63, 17)])
+def test_dgemm_tiles_agree(hlib, m, n, k):
+    """Tiles of 128 and of 64 sum in the same order: a product of many tiles and
+    the same product by blocks small enough for the small ones, bit for bit."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    rnd = lambda *s: torch.rand(*s, generator=g, dtype=torch.float64, device="cuda") - 0.5
+    ld, k2 = m + 32 - m % 32, k + k % 2
+    A, B, C0 = rnd(k, ld), rnd(n, k2), rnd(n, ld)
+    whole, parts = C0.clone(), C0.clone()
+    hlib.dgemm_sub(m, n, k, A.data_ptr(), ld, B.data_ptr(), k2, whole.data_ptr(), ld)
+    for c in range(0, n, 128):
+        w = min(128, n - c)
+        hlib.dgemm_sub(m, w, k, A.data_ptr(), ld, B.data_ptr() + 8 * c * k2, k2,
+                       parts.data_ptr() + 8 * c * ld, ld)
+    assert torch.equal(whole, parts)
+    ref = C0[:, :m] - B[:, :k] @ A[:, :m]
+    assert float((whole[:, :m] - ref).abs().max()) <= 2 * k * EPS * (1 + 0.25 * k)
+    assert torch.equal(whole[:, m:], C0[:, m:])
+
+
+@pytest.mark.parametrize("n,nb", [(4500, 256), (17000, 512), (25000, 512)])
+def test_mixed_tall_panels(hlib, n, nb):
+    """FP32 panels of 2, 4, 6 and 8 rows per thread."""
+    import torch
+
+    from rochpl_b200.hpl import Algo
+    from rochpl_b200.lib import PREC_FP16X3
+
+    x = torch.zeros(n, dtype=torch.float64, device="cuda")
+    r = hlib.pdgesv_mixed(Algo(nb, 32, 2, 2, 2, 1, 0).c(), n, x.data_ptr(), seed=5,
+                          precision=PREC_FP16X3)
+    assert r["converged"] == 1 and r["gmres_iters"] <= 10
+    assert hlib.residual_lcg(n, 5, x.data_ptr())["resid"] < 16.0
+
+
+@pytest.mark.parametrize("trans", [0, 1])
+def test_batch_getrs_with_recursive_factors(hlib, trans):
+    """Stored factors of a recursive plan: LAPACK's, whatever made them."""
+    import torch
+
+    from rochpl_b200.batch import BatchPlan
+    from rochpl_b200.lib import HPLB_BATCH_RECURSIVE
+
+    sizes, nrhs = np.array([33, 64, 97, 250], dtype=np.int32), 5
+    plan = BatchPlan(hlib, sizes, nrhs, [HPLB_BATCH_RECURSIVE] * 6)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    rnd = lambda k: torch.rand(k, generator=g, dtype=torch.float64, device="cuda") - 0.5
+    A0, B0 = rnd(plan.a_elems), rnd(plan.b_elems)
+    A, B = A0.clone(), B0.clone()
+    P = torch.zeros(plan.p_elems, dtype=torch.int32, device="cuda")
+    info = torch.zeros(plan.count, dtype=torch.int32, device="cuda")
+    plan.gesv(A.data_ptr(), B.data_ptr(), P.data_ptr(), info.data_ptr())
+    X = B0.clone()
+    plan.getrs(trans, A.data_ptr(), P.data_ptr(), X.data_ptr())
+    for n, a, b in zip(map(int, sizes), plan.a_off, plan.b_off):
+        M = A0[a:a + n * n].view(n, n).t().cpu().numpy()
+        R = B0[b:b + n * nrhs].view(nrhs, n).t().cpu().numpy()
+        ref = np.linalg.solve(M.T if trans else M, R)
+        got = X[b:b + n * nrhs].view(nrhs, n).t().cpu().numpy()
+        tol = 64 * n * EPS * np.linalg.cond(M, np.inf)
+        assert np.max(np.abs(got - ref)) / np.max(np.abs(ref)) <= tol
+    plan.close()
