@@ -99,12 +99,15 @@ hplb_status hplb_set_stream(hplb_ctx* ctx, void* stream);
 /* Per-context options (no counterpart in the reference).
  *   HPLB_OPT_LEAF: where the panel leaf keeps the rows of its NBMIN-wide slice
  *   while it factors it -- HPLB_LEAF_AUTO (default: in the registers of one
- *   thread-block cluster of up to 16 SMs when the slice fits there, else in
+ *   thread-block cluster of up to 16 SMs, which then factors the whole panel
+ *   (panels of up to 32768 rows, NB <= 1024, NBMIN <= 32); else as one launch
+ *   per step, in a cluster's registers when the slice fits there, else in
  *   registers across the GPU, else shared memory, else global memory),
  *   HPLB_LEAF_REGISTERS (registers across the GPU first, never the cluster),
  *   HPLB_LEAF_SHARED (shared memory first) or HPLB_LEAF_GLOBAL.  All perform
- *   the same operations in the same order and give identical results; the
- *   choice only moves time.  The rocHPL leaf keeps its slice in global memory
+ *   the same operations in the same order and give identical results (the
+ *   default splits the leaves of panels above 12288 rows, which rounds
+ *   differently there); the choice only moves time.  The rocHPL leaf keeps its slice in global memory
  *   (src/pfact/HPL_pdpanrlT_device.cpp:23-320). */
 #define HPLB_OPT_LEAF 1
 #define HPLB_LEAF_AUTO 0

@@ -5,26 +5,34 @@
 //
 // What bounds it: a panel is a chain of NB pivot searches over all its rows,
 // so it is latency-bound, and beside the trailing update it also waits for SMs
-// at every launch.  Hence one launch per panel instead of about 3 NB / NBMIN
-// (N = 16384, NB = 512: 46), the cluster's SMs held from start to end, and a
-// column step built around one one-way message:
-//   * the leaf's rows live in registers (RPT rows of W columns per thread); the
-//     columns are reached at compile-time positions, eight columns of code per
-//     pass, the registers rotated by eight columns between passes;
+// at every launch.  Hence one launch for a whole run of the recursion's
+// operations (N = 16384, NB = 512: 5 to 8 launches per panel instead of 46), the
+// cluster's SMs held from start to end, and a column step built around one
+// one-way message:
+//   * the leaf's rows live in registers (RPT rows of W columns per thread), the
+//     current column always in register 0: the update writes each column one
+//     register down, so one short loop body serves every column (eight unrolled
+//     bodies spent a third of their time fetching instructions); finished
+//     columns wait in shared memory;
 //   * rows never move while the leaf is factored: each thread tracks the
 //     position its row has under the interchanges and writes it there at the
 //     end, so no diagonal row is exchanged;
-//   * every CTA pushes its candidate row (W values, its position, the
-//     reciprocal of its pivot) into every CTA's shared memory with st.async,
-//     whose arrival completes the receiver's mbarrier: no cluster barrier and
-//     no remote read per column, the search for the winner is local;
+//   * every CTA pushes its candidate row (the columns from the current one on,
+//     and its position) into every CTA's shared memory with st.async, whose
+//     arrival completes the receiver's mbarrier: no cluster barrier and no
+//     remote read per column, the search for the winner is local;
 //   * only column k + 1 is updated before the next candidate is published; the
 //     remaining columns are updated while the messages travel (the published
-//     row's share is done by the publishing warp, one lane per column).
+//     row's share is done by the publishing warp, two columns per lane).
 // Between the leaves, the recursion's U12 = L11^-1 A12 (a warp per column,
 // blocked substitution with inverted 32 x 32 diagonal blocks) and
 // A22 -= L21 U12 (DMMA m16n8k8 in FP64, FFMA in FP32, a share of the rows per
 // CTA, cp.async-staged), separated by cluster barriers.
+//
+// Measured on one B200: a column step 2.7 us (one launch per leaf, 4096 rows)
+// -> 1.2 us, of which about 0.45 us is staging and sending the candidate, 0.3 us
+// its way to the other CTAs and the rest the search and the updates' latency; a
+// panel of 4096 x 256 about 1.1 ms -> 0.55 ms, of 8192 x 512 in FP32 3.7 -> 1.3 ms.
 //
 // Every operation is the one of the launch-per-step path (panel.cu, dgemm_tma.cu,
 // sgemm.cu) in the same order per element, so both give identical bits; leaves
@@ -1316,7 +1324,9 @@ cudaError_t launch_form(FusedParams<T>& P, int g, cudaStream_t stream, bool* don
 }
 
 // Rows per thread and leaf width by the rows a cluster of 16 must hold: the
-// widest leaf whose RPT x W values stay within 192 of a thread's registers.
+// widest leaf whose RPT x W values stay within 192 of a thread's registers.  A
+// narrower leaf costs an update and its barriers more per 32 columns (12288 rows
+// as one leaf of 32: 76 us, 16384 rows as two of 16: 111 us).
 template <typename T>
 int form_width(int rows) {
   if(sizeof(T) == 8) return rows <= 12288 ? 32 : (rows <= 24576 ? 16 : (rows <= 32768 ? 8 : 0));
@@ -1371,6 +1381,9 @@ cudaError_t launch_panel_fused(T* A, int64_t ld, int r0, int c0, int n, int jb, 
   B.rfact = rfact;
   B.W     = W;
   B.rows  = rows;
+  // Products of more work than this take longer on 16 SMs than a launch over all of
+  // them with the cluster's own relaunch (8192 x 512 panel: everything in the
+  // cluster 2.43 ms FP64 and 3.54 ms FP32, with this line 1.53 and 1.76 ms).
   B.split = sizeof(T) == 8 ? 5e7 : 2.5e7;
   B.panel(0, jb);
   if(linv && !B.aligned()) B.inverses(0, jb);
@@ -1387,6 +1400,8 @@ cudaError_t launch_panel_fused(T* A, int64_t ld, int r0, int c0, int n, int jb, 
   P.dinv   = dinv;
   P.linv   = nullptr;
   P.permU  = permU;
+  // At least 64 rows per CTA (64, 128 and 256 are within 2% of each other from 100
+  // to 4096 rows, 256 is 5% slower at 500).
   const int g = cluster_for((rows + 63) / 64);
   for(size_t at = 0; at < B.ops.size();) {
     size_t end = at;
