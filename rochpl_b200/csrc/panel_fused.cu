@@ -966,24 +966,38 @@ HPLB_DEV void gemm_tiles(int m, int n, int k, const float* A, int64_t lda, const
 }
 
 // FP64: a 16 x 32 tile of the products below for a warp, straight from L2 by
-// DMMA: acc = sum over k in [k0, k1) of A(r, k) B(k, c), A column-major, B by its
-// two strides; then out(r, c) = sign * acc at out[r sr + c sc].
+// DMMA: acc = sum over k in [k0, k1) of A(r, k) B(k, c), A column-major (of a
+// strictly lower A, `step` 2, the entries k < at + r), B by its two strides; then
+// out(r, c), at out[r sr + c sc], is acc (step 0), -acc (1), out + B(at + r, c) + acc
+// (2) or out - acc (3).  What stands there already is loaded before the sum.
 HPLB_DEV void tri_warp(const double* A, int64_t lda, int mr, const double* B, int64_t sbk,
-                       int64_t sbn, int nc, int k0, int k1, double* out, int64_t sr, int64_t sc,
-                       double sign) {
+                       int64_t sbn, int nc, int k0, int k1, int step, int at, double* out,
+                       int64_t sr, int64_t sc) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
-  double    acc[4][4];
+  double    acc[4][4], old[4][4];
 #pragma unroll
   for(int j = 0; j < 4; ++j)
 #pragma unroll
-    for(int r = 0; r < 4; ++r) acc[j][r] = 0.0;
+    for(int r = 0; r < 4; ++r) {
+      const int  rr = g + (r >> 1) * 8, cc = j * 8 + 2 * t4 + (r & 1);
+      const bool in = rr < mr && cc < nc;
+      acc[j][r]     = (in && step == 2) ? __ldcg(B + (size_t)(at + rr) * sbk + (size_t)cc * sbn) : 0.0;
+      old[j][r]     = (in && step >= 2) ? __ldcg(out + (size_t)rr * sr + (size_t)cc * sc) : 0.0;
+    }
+#pragma unroll
+  for(int j = 0; j < 4; ++j)
+#pragma unroll
+    for(int r = 0; r < 4; ++r) {
+      old[j][r] += acc[j][r];
+      acc[j][r] = 0.0;
+    }
 #pragma unroll 4
   for(int k = k0; k < k1; k += 8) {
     double a[4], b[4][2];
 #pragma unroll
     for(int r = 0; r < 4; ++r) {
       const int rr = g + (r & 1) * 8, kk = k + t4 + (r >> 1) * 4;
-      a[r] = (rr < mr && kk < k1) ? __ldcg(A + (size_t)rr + (size_t)kk * lda) : 0.0;
+      a[r] = (rr < mr && kk < k1 && (step != 2 || kk < at + rr)) ? __ldcg(A + (size_t)rr + (size_t)kk * lda) : 0.0;
     }
 #pragma unroll
     for(int j = 0; j < 4; ++j)
@@ -1000,16 +1014,17 @@ HPLB_DEV void tri_warp(const double* A, int64_t lda, int mr, const double* B, in
 #pragma unroll
     for(int r = 0; r < 4; ++r) {
       const int rr = g + (r >> 1) * 8, cc = j * 8 + 2 * t4 + (r & 1);
-      if(rr < mr && cc < nc) out[(size_t)rr * sr + (size_t)cc * sc] = sign * acc[j][r];
+      if(rr < mr && cc < nc)
+        out[(size_t)rr * sr + (size_t)cc * sc] =
+            (step & 1) ? old[j][r] - acc[j][r] : old[j][r] + acc[j][r];
     }
 }
 
-// FP32: a 64 x 64 tile by a CTA: sign * sum over k in [k0, k1)
-// of A(r, k) B(k, c) to out[r sr + c sc], for r < mr and c < nc.  A column-major,
-// B by its two strides (one of them 1); k-slices of 32 through two cp.async
-// buffers (the triangular factor, B in step 0 and A in step 1, with its tile at
-// row or column `at`: what stands above its diagonal blocks is not its own and
-// counts as 0).
+// FP32: the same for a 64 x 64 tile by a CTA.  B by its two strides (one of them
+// 1); k-slices of 32 through two cp.async buffers (the triangular factor, B in
+// step 0 and A in the others, with its tile at row or column `at`: what stands
+// above its diagonal blocks, in step 2 above the strict triangle, is not its own
+// and counts as 0).
 constexpr int kTriTile = 64, kTriK = 32, kTriPa = kTriTile + 4, kTriPb = kTriK + 4;
 constexpr int kTriStage = kTriK * kTriPa + kTriTile * kTriPb;  // elements of a buffer
 
@@ -1037,12 +1052,13 @@ HPLB_DEV void tri_step(float (&acc)[16], const float* as, const float* bs) {
 }
 HPLB_DEV void tri_tile(const float* A, int64_t lda, int mr, const float* B, int64_t sbk, int64_t sbn,
                        int nc, int k0, int k1, int step, int at, float* out, int64_t sr, int64_t sc,
-                       float sign, float* sm) {
+                       float* sm) {
   auto load = [&](int kb, float* st) {
 #pragma unroll
     for(int h = 0; h < kTriTile * kTriK / kThreads; ++h) {
       const int  e = threadIdx.x + h * kThreads, r = e % kTriTile, k = e / kTriTile;
-      const bool in = r < mr && kb + k < k1 && (step == 0 || kb + k < at + r / kTri * kTri + kTri);
+      const int  end = step == 0 ? k1 : step == 2 ? at + r : at + r / kTri * kTri + kTri;
+      const bool in  = r < mr && kb + k < min(k1, end);
       cp_async1(s_addr(st + k * kTriPa + r), in ? A + (size_t)r + (size_t)(kb + k) * lda : A, in);
     }
     float* sb = st + kTriK * kTriPa;
@@ -1050,16 +1066,26 @@ HPLB_DEV void tri_tile(const float* A, int64_t lda, int mr, const float* B, int6
     for(int h = 0; h < kTriTile * kTriK / kThreads; ++h) {
       const int  e = threadIdx.x + h * kThreads;
       const int  k = sbk == 1 ? e % kTriK : e / kTriTile, c = sbk == 1 ? e / kTriK : e % kTriTile;
-      const bool in = c < nc && kb + k < k1 && (step == 1 || kb + k >= at + c / kTri * kTri);
+      const bool in = c < nc && kb + k < k1 && (step != 0 || kb + k >= at + c / kTri * kTri);
       cp_async1(s_addr(sb + c * kTriPb + k), in ? B + (size_t)(kb + k) * sbk + (size_t)c * sbn : B,
                 in);
     }
     cp_commit();
   };
-  float acc[16];
-#pragma unroll
-  for(int e = 0; e < 16; ++e) acc[e] = 0.f;
   load(k0, sm);
+  float acc[16], old[16];
+#pragma unroll
+  for(int e = 0; e < 16; ++e) {
+    const int  r = threadIdx.x % 16 * 4 + (e & 3), c = threadIdx.x / 16 * 4 + (e >> 2);
+    const bool in = r < mr && c < nc;
+    acc[e]        = (in && step == 2) ? __ldcg(B + (size_t)(at + r) * sbk + (size_t)c * sbn) : 0.f;
+    old[e]        = (in && step >= 2) ? __ldcg(out + (size_t)r * sr + (size_t)c * sc) : 0.f;
+  }
+#pragma unroll
+  for(int e = 0; e < 16; ++e) {
+    old[e] += acc[e];
+    acc[e] = 0.f;
+  }
   int buf = 0;
   for(int kb = k0; kb < k1; kb += kTriK, buf ^= 1) {
     if(kb + kTriK < k1)
@@ -1074,56 +1100,128 @@ HPLB_DEV void tri_tile(const float* A, int64_t lda, int mr, const float* B, int6
 #pragma unroll
   for(int e = 0; e < 16; ++e) {
     const int r = threadIdx.x % 16 * 4 + (e & 3), c = threadIdx.x / 16 * 4 + (e >> 2);
-    if(r < mr && c < nc) out[(size_t)r * sr + (size_t)c * sc] = sign * acc[e];
+    if(r < mr && c < nc)
+      out[(size_t)r * sr + (size_t)c * sc] = (step & 1) ? old[e] - acc[e] : old[e] + acc[e];
+  }
+}
+
+// Inverses of the kSubst x kSubst diagonal blocks of L into X by substitution on
+// the identity with L's inverted 32 x 32 diagonal blocks, CP neighbouring columns a
+// warp.
+constexpr int kSubst = 256;
+constexpr size_t kInverseBytes = (size_t)kWarps * 4 * kSubst * sizeof(double);
+static_assert(kInverseBytes >= 2 * kTriStage * sizeof(float), "tri_tile's buffers");
+template <typename T, int CP>
+HPLB_DEV void invert_by_substitution(const T* L, int64_t ldl, int jb, const T* dinv, T* X,
+                                     int64_t ldx, int gw, int nw, T* sm) {
+  const int lane = threadIdx.x & 31;
+  T*        x    = sm + (size_t)(threadIdx.x >> 5) * CP * kSubst;  // by column, rows of the block
+  for(int c = gw * CP; c < jb; c += nw * CP) {
+    const int base = c / kSubst * kSubst, m = min(kSubst, jb - base);
+    const int first = (c - base) / kTri * kTri;  // the columns' own 32 rows
+    for(int row0 = first; row0 < m; row0 += kTri) {
+      const int r = base + row0 + lane;
+      const T*  d = dinv + (size_t)(base + row0) / kTri * kTri * kTri;
+      T         v[CP];
+      if(row0 == first) {
+#pragma unroll
+        for(int q = 0; q < CP; ++q) v[q] = __ldcg(d + (c % kTri + q) * kTri + lane);
+      } else {
+        T dv[kTri];
+#pragma unroll
+        for(int k = 0; k < kTri; ++k) dv[k] = row0 + k < m ? __ldcg(d + k * kTri + lane) : (T)0;
+#pragma unroll
+        for(int q = 0; q < CP; ++q) v[q] = (T)0;
+        for(int k = first; k < row0; k += 16) {
+          T lv[16];
+#pragma unroll
+          for(int t = 0; t < 16; ++t)
+            lv[t] = r < jb ? __ldcg(L + (size_t)r + (size_t)(base + k + t) * (size_t)ldl) : (T)0;
+#pragma unroll
+          for(int t = 0; t < 16; ++t)
+#pragma unroll
+            for(int q = 0; q < CP; ++q) v[q] = fma_(-lv[t], x[q * kSubst + k + t], v[q]);
+        }
+#pragma unroll
+        for(int q = 0; q < CP; ++q) x[q * kSubst + row0 + lane] = r < jb ? v[q] : (T)0;
+        __syncwarp();
+#pragma unroll
+        for(int q = 0; q < CP; ++q) v[q] = (T)0;
+#pragma unroll
+        for(int k = 0; k < kTri; ++k)
+#pragma unroll
+          for(int q = 0; q < CP; ++q) v[q] = fma_(dv[k], x[q * kSubst + row0 + k], v[q]);
+        __syncwarp();
+      }
+#pragma unroll
+      for(int q = 0; q < CP; ++q) {
+        x[q * kSubst + row0 + lane] = v[q];
+        if(r < jb && c + q < jb) X[(size_t)r + (size_t)(c + q) * (size_t)ldx] = v[q];
+      }
+      __syncwarp();
+    }
   }
 }
 
 // X (jb x jb, leading dimension ldx) = L^-1 for the unit-lower L at L, from its
-// inverted 32 x 32 diagonal blocks, by doubling: for neighbouring blocks of s
-// columns, [A 0; B C]^-1 = [A^-1 0; -C^-1 B A^-1, C^-1], each product a tile per
-// warp (FP64) or CTA (FP32, whose FFMA loop wants its operands in shared memory:
-// 197 us at jb = 512 with warp tiles, 68 with these).  log2(jb / 32) levels of two products and two cluster barriers instead
-// of a chain of jb / 32 substitution steps, which the blocked substitution on
-// the identity needs.  B A^-1 waits, transposed, in X's block above the diagonal.
+// inverted 32 x 32 diagonal blocks: blocks of kSubst columns by substitution, wider
+// ones by doubling: for neighbouring blocks of s columns, [A 0; B C]^-1 =
+// [A^-1 0; X21 C^-1] with X21 = -C^-1 T, T = B A^-1, each product a tile per warp
+// (FP64) or CTA (FP32, whose FFMA loop wants its operands in shared memory).  T
+// waits, transposed, in X's block above the diagonal.
+//
+// The rounding of T and of the product meets C again in L X - I, the residual that
+// U12 = L11^-1 A12 sees, and grows with |C| |C^-1|; substitution has no such growth.
+// Hence X21 -= C^-1 (T + C X21), which brings the residual back to substitution's.
+// LCG panels of 2048 rows, FP64, |L X - I| / eps in the Frobenius norm and time:
+//   jb = 256  this 274, 34 us;  doubling from 32 on, uncorrected 726, 39 us
+//   jb = 512  this 721, 118 us;  doubling 3744, 77 us;  substitution alone 688, 171 us
+// (kSubst = 128 takes 51 and 128 us: each product step is a few us of latency.)
 template <typename T>
 HPLB_DEV void lower_inverse(const T* L, int64_t ldl, int jb, const T* dinv, T* X, int64_t ldx,
                             unsigned G, unsigned me, T* sm) {
   const int gw = (int)me + (int)G * (int)(threadIdx.x >> 5), nw = (int)G * kWarps;
   const int lane = threadIdx.x & 31;
-  for(int c = gw; c < jb; c += nw) {
-    const int r = c / kTri * kTri + lane;
-    if(r < jb)
-      X[(size_t)r + (size_t)c * ldx] =
-          __ldcg(dinv + (size_t)(c / kTri) * kTri * kTri + (c % kTri) * kTri + lane);
-  }
-  for(int s = kTri; s < jb; s *= 2) {
+  // Columns per warp: as few passes as four at once allow.
+  if(jb <= nw)
+    invert_by_substitution<T, 1>(L, ldl, jb, dinv, X, ldx, gw, nw, sm);
+  else if(jb <= 2 * nw)
+    invert_by_substitution<T, 2>(L, ldl, jb, dinv, X, ldx, gw, nw, sm);
+  else
+    invert_by_substitution<T, 4>(L, ldl, jb, dinv, X, ldx, gw, nw, sm);
+  for(int s = kSubst; s < jb; s *= 2) {
     constexpr bool wide = sizeof(T) == 4;
     constexpr int  TR = wide ? kTriTile : 16, TC = wide ? kTriTile : 32;
     const int      tr = (s + TR - 1) / TR, tc = (s + TC - 1) / TC;
     const int      units = (jb + 2 * s - 1) / (2 * s) * tr * tc;
-    for(int step = 0; step < 2; ++step) {
+    // Step 0: T = B A^-1.  1: X21 = -C^-1 T.  2: T += C X21 (X21 itself and the
+    // strict triangle of L's C).  3: X21 -= C^-1 T.
+    for(int step = 0; step < 4; ++step) {
       cluster_sync();
       for(int e = wide ? (int)me : gw; e < units; e += wide ? (int)G : nw) {
         const int base = e / (tr * tc) * 2 * s, r = e / tc % tr * TR, c = e % tc * TC;
         const int s2 = min(s, jb - base - s), mr = s2 - r;
         if(mr <= 0) continue;
-        T*       bt = X + (size_t)base + (size_t)(base + s) * ldx;  // (B A^-1)^T
-        const T* A  = step == 0 ? L + (size_t)(base + s + r) + (size_t)base * ldl
-                                : X + (size_t)(base + s + r) + (size_t)(base + s) * ldx;
-        const T* B  = step == 0 ? X + (size_t)base + (size_t)(base + c) * ldx : bt + c;
-        T* out = step == 0 ? bt + (size_t)c + (size_t)r * ldx
-                           : X + (size_t)(base + s + r) + (size_t)(base + c) * ldx;
-        const int64_t lda = step == 0 ? ldl : ldx, sbk = step == 0 ? 1 : ldx,
-                      sbn = step == 0 ? ldx : 1;
+        const bool to_t = (step & 1) == 0;
+        const int  low  = base + s;                           // C's first row
+        T*         bt   = X + (size_t)base + (size_t)low * ldx;  // T^t
+        const T* A = step == 0   ? L + (size_t)(low + r) + (size_t)base * ldl
+                     : step == 2 ? L + (size_t)(low + r) + (size_t)low * ldl
+                                 : X + (size_t)(low + r) + (size_t)low * ldx;
+        const T* B = step == 0   ? X + (size_t)base + (size_t)(base + c) * ldx
+                     : step == 2 ? X + (size_t)low + (size_t)(base + c) * ldx
+                                 : bt + c;
+        T* out = to_t ? bt + (size_t)c + (size_t)r * ldx
+                      : X + (size_t)(low + r) + (size_t)(base + c) * ldx;
+        const int64_t lda = to_t ? ldl : ldx, sbk = to_t ? 1 : ldx, sbn = to_t ? ldx : 1;
         // The triangular factor's columns from the tile's on, rows up to its last.
         const int k0 = step == 0 ? c / kTri * kTri : 0;
         const int k1 = step == 0 ? s : min(s2, (r + TR + kTri - 1) / kTri * kTri);
-        const T   sign = step == 0 ? (T)1 : (T)-1;
+        const int at = step == 0 ? c : r;
         if constexpr(wide)
-          tri_tile(A, lda, mr, B, sbk, sbn, s - c, k0, k1, step, step == 0 ? c : r, out, sbn, sbk,
-                   sign, sm);
+          tri_tile(A, lda, mr, B, sbk, sbn, s - c, k0, k1, step, at, out, sbn, sbk, sm);
         else
-          tri_warp(A, lda, mr, B, sbk, sbn, s - c, k0, k1, out, sbn, sbk, sign);
+          tri_warp(A, lda, mr, B, sbk, sbn, s - c, k0, k1, step, at, out, sbn, sbk);
       }
     }
   }
@@ -1146,7 +1244,7 @@ constexpr size_t dyn_bytes() {
   b = at_least(b, (size_t)GemmCfg<T>::stages(1) * GemmCfg<T>::stage(1) * sizeof(T));
   b = at_least(b, (size_t)GemmCfg<T>::stages(2) * GemmCfg<T>::stage(2) * sizeof(T));
   b = at_least(b, (size_t)GemmCfg<T>::stages(4) * GemmCfg<T>::stage(4) * sizeof(T));
-  b = at_least(b, (size_t)2 * kTriStage * sizeof(float));
+  b = at_least(b, kInverseBytes);
   b = at_least(b, (size_t)kWarps * 2 * (kMaxNb + 1) * sizeof(T));           // trsm_cols<T, 2>
   return at_least(b, (size_t)kWarps * kTri * kTopPitch * sizeof(T));        // invert_blocks
 }
@@ -1220,6 +1318,7 @@ panel_fused_kernel(const __grid_constant__ FusedParams<T> P) {
       }
       P.permU[e] = fwd ? (at >= P.jb ? at : -1) : at;
     }
+    __syncthreads();  // s_piv is read: its memory is the inverse's now
   }
   lower_inverse<T>(P.A + (size_t)P.r0 + (size_t)P.c0 * (size_t)P.ld, P.ld, P.jb, P.dinv, P.linv,
                    P.jb, G, me, sm);
@@ -1439,7 +1538,7 @@ cudaError_t launch_unit_lower_inverse(const T* L, int64_t ldl, int jb, const T* 
   static signed char placeable[kMaxG + 1] = {};
   for(int g = cluster_for((jb + 31) / 32); g > 0; g /= 2) {
     bool              done = false;
-    const cudaError_t e    = launch_cluster(lower_inverse_kernel<T>, g, 2 * kTriStage * sizeof(float),
+    const cudaError_t e    = launch_cluster(lower_inverse_kernel<T>, g, kInverseBytes,
                                             placeable, stream, &done,
                                             L, ldl, jb, dinv, Linv, ldinv);
     if(done || e != cudaSuccess) return e;

@@ -63,6 +63,87 @@ def test_panel_zero_pivot(hlib, oracle):
         assert _panel(hlib, oracle, n, 64, 32, 2, LEAF_AUTO, zero_col=37)[2] == 38
 
 
+def _unit_lower(hlib, oracle, jb):
+    """The factored LCG panel of 2048 rows and its unit-lower block."""
+    import torch
+
+    from rochpl_b200.hpl import Algo
+
+    n = 2048
+    ld = oracle.default_ld(n)
+    W = torch.zeros((2 * jb, ld), dtype=torch.float64, device="cuda")
+    hlib.matgen_block(n, n, 0, 0, n, jb, 7, W.data_ptr(), ld)
+    piv = torch.zeros(jb, dtype=torch.int32, device="cuda")
+    assert hlib.panel_factor(Algo(jb, min(32, jb), 2, 2, 2, 1, 0).c(), n, 0, jb, W.data_ptr(),
+                             ld, 0, piv.data_ptr()) == 0
+    return n, ld, W, np.tril(W[:jb, :jb].cpu().numpy().T, -1) + np.eye(jb)
+
+
+def _residual(L, X):
+    """|L X - I| in the Frobenius norm; X has L's shape."""
+    assert np.array_equal(np.triu(X, 1), np.zeros_like(X))
+    wide = np.float64 if X.dtype == np.float32 else np.longdouble
+    return float(np.linalg.norm((L.astype(wide) @ X.astype(wide) - np.eye(len(L))).astype(float)))
+
+
+# L11^-1 leaves no larger a residual L X - I, which is what U12 = L11^-1 A12 sees,
+# than the blocked substitution on the identity.  Both are norms of jb^2 / 2
+# rounding errors of the same size, so they agree closely (seen: 0.98 to 1.05 of
+# it); doubling without a correction is at 1.5 times at jb = 128 and 5 at 512.
+SLACK = 1.25
+
+
+@pytest.mark.parametrize("jb", [33, 64, 65, 128, 200, 255, 257, 400, 511])
+def test_unit_lower_inverse_residual(hlib, oracle, jb):
+    """hplb_panel_update on the identity against hplb_laswp_trsm on it."""
+    import torch
+
+    n, ld, W, L = _unit_lower(hlib, oracle, jb)
+    eye = torch.eye(jb, dtype=torch.float64, device="cuda")
+    X = torch.zeros((jb, ld), dtype=torch.float64, device="cuda")
+    X[:, :jb] = eye
+    W[jb:, :jb] = eye
+    own = torch.arange(jb, dtype=torch.int32, device="cuda")  # no interchanges
+    hlib.panel_update(n, 0, jb, W.data_ptr(), ld, own.data_ptr(), X.data_ptr(), ld, 0, jb)
+    hlib.laswp_trsm(W.data_ptr(), ld, 0, jb, 0, range(jb), jb, jb)
+    new, sub = (_residual(L, T[:, :jb].cpu().numpy().T) for T in (X, W[jb:]))
+    assert new <= SLACK * sub, (new / EPS, sub / EPS)
+
+
+@pytest.mark.parametrize("jb", [96, 256, 300, 512])
+def test_unit_lower_inverse_residual_fp32(hlib, oracle, jb):
+    """The mixed form's FP32 inverse, called by its C++ symbol, against the
+    substitution in FP32 on the host."""
+    import ctypes
+
+    import torch
+
+    _, _, _, L = _unit_lower(hlib, oracle, jb)
+    L = L.astype(np.float32)
+    dL = torch.from_numpy(np.ascontiguousarray(L.T)).cuda()
+    dinv = torch.zeros((jb // 32 + 1) * 1024, dtype=torch.float32, device="cuda")
+    X = torch.full((jb, jb), np.nan, dtype=torch.float32, device="cuda")
+    P, q, i = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int
+    sym = "_ZN4hplb{}IfEE9cudaError{}P11CUstream_st"
+    diag = getattr(hlib.L, sym.format("15launch_diag_inv", "PKT_liiiPS2_"))
+    diag.argtypes = [P, q, i, i, i, P, P]
+    inv = getattr(hlib.L, sym.format("25launch_unit_lower_inverse", "PKT_liS4_PS2_l"))
+    inv.argtypes = [P, q, i, P, P, q, P]
+    torch.cuda.synchronize()
+    assert diag(dL.data_ptr(), jb, 0, 0, jb, dinv.data_ptr(), None) == 0
+    assert inv(dL.data_ptr(), jb, jb, dinv.data_ptr(), X.data_ptr(), jb, None) == 0
+    torch.cuda.synchronize()
+    ref = np.eye(jb, dtype=np.float32)
+    for b in range(0, jb, 32):  # 32 rows by their block's inverse, as on the GPU
+        e = min(b + 32, jb)
+        D = np.eye(e - b, dtype=np.float32)
+        for r in range(1, e - b):
+            D[r] -= L[b + r, b:b + r] @ D[:r]
+        ref[b:e] = D @ (ref[b:e] - L[b:e, :b] @ ref[:b])
+    new, sub = _residual(L, X.cpu().numpy().T), _residual(L, ref)
+    assert new <= SLACK * sub, (new * 2 ** 24, sub * 2 ** 24)
+
+
 @pytest.mark.parametrize("n,nb,nrhs", [(1, 1, 1), (63, 64, 7), (64, 64, 8), (65, 64, 9),
                                        (130, 65, 33), (200, 200, 31), (257, 48, 40),
                                        (300, 33, 128), (300, 64, 129)])
