@@ -168,7 +168,7 @@ hplb_status hplb_pdgesv(hplb_ctx* ctx, const hplb_algo* algo, int n, double* dA,
  * ld >= n, n + nrhs columns) and takes every interchange and trailing update
  * as HPL_pdgesv's column n does, so no separate forward solve is needed; then
  * X = U^-1 B (device, n x nrhs, leading dimension ldx >= n) by a persistent
- * back-solve of 32 right-hand sides per launch.  dA, ipiv_out and info as in
+ * back-solve of 128 right-hand sides per launch.  dA, ipiv_out and info as in
  * hplb_pdgesv; nrhs = 1 gives the same result as hplb_pdgesv.  The reference
  * carries exactly one right-hand side (include/hpl_pgesv.hpp:162). */
 hplb_status hplb_gesv(hplb_ctx* ctx, const hplb_algo* algo, int n, int nrhs, double* dA,

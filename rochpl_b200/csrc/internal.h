@@ -116,14 +116,14 @@ cudaError_t launch_col_rank1(double* A, int64_t ld, int r0, int r1, int c0, int 
                              double piv, const double* u, int num_sms, cudaStream_t stream);
 // X (n x nrhs, leading dimension ldx) = U^-1 Y for the upper triangle of A
 // (n x n, leading dimension ld); Y (leading dimension ldy) may be X itself.
-// Persistent, one launch per 32 right-hand sides; flags: trsv_flag_ints(n).
+// Persistent, one launch per 128 right-hand sides; flags: trsv_flag_ints(n).
 cudaError_t launch_trsm_upper(const double* A, int64_t ld, int n, int nrhs, const double* Y,
                               int64_t ldy, double* X, int64_t ldx, int* flags, int* status,
                               cudaStream_t stream, int* launches);
 // X (rows x nrhs) <- L^-1 X for the unit-lower ns x ns L in the first ns rows, and
-// X -= L21 X_top in the rows - ns below, in one persistent launch per 32
+// X -= L21 X_top in the rows - ns below, in one persistent launch per 128
 // right-hand sides; flags: trsv_flag_ints(ns), zeroed by the call, or that many for
-// each 32 right-hand sides, zeroed by the caller.
+// each 128 right-hand sides, zeroed by the caller.
 cudaError_t launch_trsm_lower(const double* L, int64_t ldl, int ns, int rows, int nrhs, double* X,
                               int64_t ldx, int* flags, int* status, bool zeroed,
                               cudaStream_t stream, int* launches);

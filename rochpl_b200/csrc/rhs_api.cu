@@ -11,7 +11,7 @@
 // and
 //   A^-T = P_0^T E_0^T ... P_{np-1}^T E_{np-1}^T U^-T.
 // Up to 128 right-hand sides a panel's L11 and the rows below it take one
-// persistent launch per 32 of them (launch_trsm_lower): with a CTA per column for
+// persistent launch (launch_trsm_lower): with a CTA per column for
 // L11 and a product kernel for the rows below, the chain of launches bounded the
 // solve (N = 8192, NB = 512, 32 right-hand sides: 4.25 ms, now 1.69).  More
 // right-hand sides take the blocked substitution and DMMA GEMMs (explicit
@@ -39,10 +39,8 @@ struct Rhs {
   int*          perm;
   cudaStream_t  st;
 
-  // Flags of one panel's lower solves.
-  static size_t panel_flags(int nb, int nrhs) {
-    return trsv_flag_ints(nb) * (size_t)((nrhs + 31) / 32);
-  }
+  // Flags of one panel's lower solve.
+  static size_t panel_flags(int nb) { return trsv_flag_ints(nb); }
   static size_t ws_doubles(int n, int nb, int nrhs) {
     const size_t nblk = (size_t)nb / 32 + 1;
     return (size_t)nb * nrhs + (size_t)nb * nb + nb + nblk * 1024 + 64 +
@@ -103,14 +101,14 @@ struct Rhs {
     hplb_status s;
     if(nrhs <= 128)  // the flags of every panel's launches at once
       CK(cudaMemsetAsync(ctx->d_trsv, 0,
-                         panel_flags(nb, nrhs) * ((n + nb - 1) / nb) * sizeof(int), st));
+                         panel_flags(nb) * ((n + nb - 1) / nb) * sizeof(int), st));
     for(int j = 0; j < n; j += nb) {
       const int jb = std::min(nb, n - j);
       CK(launch_permute_rows(B, ldb, j, jb, panel_perm(j), nrhs, st));
       ctx->launches += 1;
-      if(nrhs <= 128) {  // L11^-1 and the rows below in one launch per 32 right-hand sides
+      if(nrhs <= 128) {  // L11^-1 and the rows below in one launch
         CK(launch_trsm_lower(lu(j, j), ld, jb, n - j, nrhs, b(j), ldb,
-                             ctx->d_trsv + panel_flags(nb, nrhs) * (size_t)(j / nb), ctx->d_status,
+                             ctx->d_trsv + panel_flags(nb) * (size_t)(j / nb), ctx->d_status,
                              true, st, &ctx->launches));
         continue;
       }
@@ -118,7 +116,7 @@ struct Rhs {
       CK(update(n - j - jb, jb, lu(j + jb, j), ld, b(j), ldb, b(j + jb), ldb));
       ctx->launches += 1;
     }
-    if(nrhs <= 128) {  // U X = Y in one persistent launch per 32 right-hand sides
+    if(nrhs <= 128) {  // U X = Y in one persistent launch
       CK(launch_trsm_upper(LU, ld, n, nrhs, B, ldb, B, ldb, ctx->d_trsv, ctx->d_status, st,
                            &ctx->launches));
       return HPLB_OK;
@@ -200,7 +198,7 @@ hplb_status hplb_getrs(hplb_ctx* ctx, int trans, int n, int nb, int nrhs, const 
                2 * (size_t)R.nb * ((n + R.nb - 1) / R.nb))) != HPLB_OK)
     return s;
   if(trans && (s = grow(ctx, &ctx->r_t, &ctx->r_t_cap, (size_t)R.ldt * n)) != HPLB_OK) return s;
-  const size_t flags = R.nrhs <= 128 ? Rhs::panel_flags(R.nb, nrhs) * ((n + R.nb - 1) / R.nb) : 0;
+  const size_t flags = R.nrhs <= 128 ? Rhs::panel_flags(R.nb) * ((n + R.nb - 1) / R.nb) : 0;
   if((s = grow(ctx, &ctx->d_trsv, &ctx->trsv_cap, std::max(flags, trsv_flag_ints(n)))) != HPLB_OK)
     return s;
   R.carve(ctx->r_ws);

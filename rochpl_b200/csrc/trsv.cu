@@ -197,10 +197,12 @@ trsv_kernel(const double* __restrict__ A, int64_t ld, int n, const double* __res
 // store, flag.  Eight right-hand sides per CTA (four CTAs share a tile through
 // L2) and the tensor-core products keep that chain short: the earlier form, 32
 // right-hand sides per CTA with FMA loops bound by shared-memory loads, took
-// 12.3 us per row block (N = 8192: 1576 us, now 424 us).  Waits are bounded
-// (status site 42).  X may alias Y: a block of Y is read only by its own CTA,
+// 12.3 us per row block (N = 8192: 1576 us, now 424 us).  Up to 128 right-hand sides
+// run in one launch, their groups' chains beside each other; a launch per 32 was as
+// many chains in turn (hplb_getrs, 64 right-hand sides, N = 1000, NB = 64: plain 1.30,
+// transposed 3.20 ms, now 0.73 and 2.16).  Waits are bounded (status site 42).  X may alias Y: a block of Y is read only by its own CTA,
 // before that CTA writes X there.
-constexpr int kNr       = 32;       // right-hand sides per launch
+constexpr int kNr       = 128;      // right-hand sides per launch
 constexpr int kNg       = 8;        // right-hand sides per CTA
 constexpr int kTp       = kTb + 4;  // pitch = 4 mod 16: fragment loads free of conflicts
 constexpr int kTrsmSite = 42;

@@ -168,6 +168,29 @@ def test_getrs_block_edges(hlib, oracle, n, nb, nrhs, trans):
     assert err <= tol, (err, tol)
 
 
+@pytest.mark.parametrize("trans", [0, 1])
+def test_getrs_launches_do_not_grow_with_right_hand_sides(hlib, oracle, trans):
+    """Up to 128 right-hand sides a triangular solve is one launch: a chain of row
+    blocks per 32 of them in turn made 64 take 1.5 to 1.8 times as long."""
+    import torch
+
+    from rochpl_b200.hpl import Algo
+
+    n, nb = 300, 64
+    M = oracle.matgen(n, n + 128, 11)
+    LU = torch.from_numpy(np.ascontiguousarray(M[:n, :n].T)).cuda()
+    piv = torch.zeros(n, dtype=torch.int32, device="cuda")
+    hlib.getrf(Algo(nb, 16, 2, 2, 2, 1, 0).c(), n, LU.data_ptr(), n, piv.data_ptr())
+    launches, cols = [], []
+    for nrhs in (8, 33, 64, 128):
+        X = torch.from_numpy(np.ascontiguousarray(M[:n, n:n + nrhs].T)).cuda()
+        hlib.getrs(trans, n, nb, nrhs, LU.data_ptr(), n, piv.data_ptr(), X.data_ptr(), n)
+        launches.append(hlib.last_timing()["kernel_launches"])
+        cols.append(X[:8].clone())
+    assert len(set(launches)) == 1, launches
+    assert all(torch.equal(c, cols[0]) for c in cols)  # a group's sums are its own
+
+
 @pytest.mark.parametrize("n", [1, 255, 257, 512, 2047, 2049])
 def test_residual_pass_edges(hlib, oracle, n):
     """One read of the stored matrix: the regenerated check's bits, the oracle's
