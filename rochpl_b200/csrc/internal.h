@@ -122,11 +122,10 @@ cudaError_t launch_trsm_upper(const double* A, int64_t ld, int n, int nrhs, cons
                               cudaStream_t stream, int* launches);
 // X (rows x nrhs) <- L^-1 X for the unit-lower ns x ns L in the first ns rows, and
 // X -= L21 X_top in the rows - ns below, in one persistent launch per 128
-// right-hand sides; flags: trsv_flag_ints(ns), zeroed by the call, or that many for
-// each 128 right-hand sides, zeroed by the caller.
+// right-hand sides; flags: trsv_flag_ints(ns) for each, zeroed by the caller.
 cudaError_t launch_trsm_lower(const double* L, int64_t ldl, int ns, int rows, int nrhs, double* X,
-                              int64_t ldx, int* flags, int* status, bool zeroed,
-                              cudaStream_t stream, int* launches);
+                              int64_t ldx, int* flags, int* status, cudaStream_t stream,
+                              int* launches);
 cudaError_t launch_gemv_acc(int m, int k, const double* U, int64_t ld, const double* x,
                             double* z, cudaStream_t stream);
 cudaError_t launch_vsub(int n, const double* y, const double* s, double* r, cudaStream_t stream);

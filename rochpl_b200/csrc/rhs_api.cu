@@ -37,10 +37,20 @@ struct Rhs {
   double *      W, *M1, *dvec, *dinv, *T, *SK;  // SK: split-k partial products
   int64_t       ldt;  // rows of T: n rounded up to 16, + 16, so a 16-row slab never leaves it
   int*          perm;
+  int*          flags;  // of the next panel's lower solve
   cudaStream_t  st;
 
-  // Flags of one panel's lower solve.
-  static size_t panel_flags(int nb) { return trsv_flag_ints(nb); }
+  // Flags of the lower solves: one per panel, two in the transposed solve.
+  static size_t all_flags(int n, int nb, bool trans) {
+    return trsv_flag_ints(nb) * (size_t)((n + nb - 1) / nb) * (trans ? 2 : 1);
+  }
+  // X <- L^-1 X of a panel and the rows below it (launch_trsm_lower), nrhs <= 128.
+  cudaError_t lower(const double* L, int64_t ldl, int jb, int rows, double* X, int64_t ldx) {
+    int* f = flags;
+    flags += trsv_flag_ints(nb);
+    return launch_trsm_lower(L, ldl, jb, rows, nrhs, X, ldx, f, ctx->d_status, st,
+                             &ctx->launches);
+  }
   static size_t ws_doubles(int n, int nb, int nrhs) {
     const size_t nblk = (size_t)nb / 32 + 1;
     return (size_t)nb * nrhs + (size_t)nb * nb + nb + nblk * 1024 + 64 +
@@ -65,8 +75,7 @@ struct Rhs {
   hplb_status trsm(double* X, int64_t ldx, int jb, const double* L, int64_t ldl) {
     hplb_ctx* ctx = this->ctx;
     if(nrhs <= 128) {
-      CK(launch_trsm_lower(L, ldl, jb, jb, nrhs, X, ldx, ctx->d_trsv, ctx->d_status, false, st,
-                           &ctx->launches));
+      CK(lower(L, ldl, jb, jb, X, ldx));
       return HPLB_OK;
     }
     CK(launch_diag_inv<double>(L, ldl, 0, 0, jb, dinv, st));
@@ -99,17 +108,12 @@ struct Rhs {
   hplb_status solve() {
     hplb_ctx*   ctx = this->ctx;
     hplb_status s;
-    if(nrhs <= 128)  // the flags of every panel's launches at once
-      CK(cudaMemsetAsync(ctx->d_trsv, 0,
-                         panel_flags(nb) * ((n + nb - 1) / nb) * sizeof(int), st));
     for(int j = 0; j < n; j += nb) {
       const int jb = std::min(nb, n - j);
       CK(launch_permute_rows(B, ldb, j, jb, panel_perm(j), nrhs, st));
       ctx->launches += 1;
       if(nrhs <= 128) {  // L11^-1 and the rows below in one launch
-        CK(launch_trsm_lower(lu(j, j), ld, jb, n - j, nrhs, b(j), ldb,
-                             ctx->d_trsv + panel_flags(nb) * (size_t)(j / nb), ctx->d_status,
-                             true, st, &ctx->launches));
+        CK(lower(lu(j, j), ld, jb, n - j, b(j), ldb));
         continue;
       }
       if((s = trsm(b(j), ldb, jb, lu(j, j), ld)) != HPLB_OK) return s;
@@ -198,9 +202,10 @@ hplb_status hplb_getrs(hplb_ctx* ctx, int trans, int n, int nb, int nrhs, const 
                2 * (size_t)R.nb * ((n + R.nb - 1) / R.nb))) != HPLB_OK)
     return s;
   if(trans && (s = grow(ctx, &ctx->r_t, &ctx->r_t_cap, (size_t)R.ldt * n)) != HPLB_OK) return s;
-  const size_t flags = R.nrhs <= 128 ? Rhs::panel_flags(R.nb) * ((n + R.nb - 1) / R.nb) : 0;
+  const size_t flags = nrhs <= 128 ? Rhs::all_flags(n, R.nb, trans != 0) : 0;
   if((s = grow(ctx, &ctx->d_trsv, &ctx->trsv_cap, std::max(flags, trsv_flag_ints(n)))) != HPLB_OK)
     return s;
+  R.flags = ctx->d_trsv;
   R.carve(ctx->r_ws);
   R.perm = ctx->r_perm;
   R.T    = ctx->r_t;
@@ -217,6 +222,8 @@ hplb_status hplb_getrs(hplb_ctx* ctx, int trans, int n, int nb, int nrhs, const 
   ctx->launches = 0;
   cudaEvent_t e0 = next_event(ctx), e1 = next_event(ctx);
   CK(cudaEventRecord(e0, R.st));
+  // The flags of every panel's solve at once, not a memset before each.
+  if(flags > 0) CK(cudaMemsetAsync(R.flags, 0, flags * sizeof(int), R.st));
   CK(launch_perm_panels(d_ipiv, n, R.nb, R.perm, R.st));
   ctx->launches += 1;
   if((s = trans ? R.solve_t() : R.solve()) != HPLB_OK) return s;

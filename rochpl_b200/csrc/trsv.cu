@@ -86,8 +86,7 @@ HPLB_DEV void load_tile(const double* __restrict__ A, int64_t ld, int r0, int c0
 // column, left to right: column j of the inverse is -T_jj^-1 times the
 // already-inverted leading block applied to column j of U).  256 threads; T is
 // the identity from row and column kb on, which takes no step.
-template <int PITCH>
-HPLB_DEV void invert_upper(double (*T)[PITCH], int kb) {
+HPLB_DEV void invert_upper(double (*T)[kTb + 1], int kb) {
   const int t = threadIdx.x, row = t >> 2, part = t & 3;
   for(int j = 0; j < kb; ++j) {
     double s = 0.0;
@@ -200,8 +199,8 @@ trsv_kernel(const double* __restrict__ A, int64_t ld, int n, const double* __res
 // 12.3 us per row block (N = 8192: 1576 us, now 424 us).  Up to 128 right-hand sides
 // run in one launch, their groups' chains beside each other; a launch per 32 was as
 // many chains in turn (hplb_getrs, 64 right-hand sides, N = 1000, NB = 64: plain 1.30,
-// transposed 3.20 ms, now 0.73 and 2.16).  Waits are bounded (status site 42).  X may alias Y: a block of Y is read only by its own CTA,
-// before that CTA writes X there.
+// transposed 3.20 ms, now 0.73 and 2.16).  Waits are bounded (status site 42).  X may
+// alias Y: a block of Y is read only by its own CTA, before that CTA writes X there.
 constexpr int kNr       = 128;      // right-hand sides per launch
 constexpr int kNg       = 8;        // right-hand sides per CTA
 constexpr int kTp       = kTb + 4;  // pitch = 4 mod 16: fragment loads free of conflicts
@@ -232,6 +231,77 @@ HPLB_DEV void dmma(double (&d)[4], const double (&a)[4], const double (&b)[2]) {
       "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
       : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
       : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+
+// In-place inverse by a warp of the upper triangular w x w block at (o, o) of T
+// (the identity from w on), a column per lane, from the last row up: a step's row is
+// final in s[31] and the rows above it move one register up.
+template <bool UNIT>
+HPLB_DEV void invert_upper32(double (*T)[kTp], int o, int w) {
+  constexpr int kW = 32;
+  const int     lane = threadIdx.x & 31;
+  const double  d = UNIT ? 1.0 : 1.0 / T[o + lane][o + lane];
+  double        s[kW];
+#pragma unroll
+  for(int i = 0; i < kW; ++i) s[kW - 1 - i] = w - 1 - i == lane ? 1.0 : 0.0;
+  int k = w - 1;
+#pragma unroll
+  for(int half = 0; half < 2; ++half) {  // the second with half of the rows left
+#pragma unroll 1
+    for(; k >= (half == 0 ? kW / 2 : 0); --k) {
+      const double dk = UNIT ? 1.0 : __shfl_sync(0xffffffffu, d, k);
+      const double x  = lane >= k ? s[kW - 1] * dk : 0.0;
+#pragma unroll
+      for(int h = 0; h < (half == 0 ? kW : kW / 2); h += kW / 4) {
+        double u[kW / 4];
+#pragma unroll
+        for(int i = 0; i < kW / 4; ++i) u[i] = h + i < k ? T[o + k - 1 - h - i][o + k] : 0.0;
+#pragma unroll
+        for(int i = 0; i < kW / 4; ++i)
+          if(h + i < kW - 1) s[kW - 1 - h - i] = fma(-u[i], x, s[kW - 2 - h - i]);
+      }
+      T[o + k][o + lane] = x;
+    }
+  }
+}
+
+// A 16 x 8 tile per warp of the 32 x 32 product A B.
+HPLB_DEV void product32(double (&acc)[4], const double* A, const double* B) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+  const double* a = A + ((warp & 1) * 16 + g) * kTp + t4;
+  const double* b = B + t4 * kTp + (warp >> 1) * 8 + g;
+#pragma unroll
+  for(int e = 0; e < 4; ++e) acc[e] = 0.0;
+#pragma unroll
+  for(int k = 0; k < 32; k += 8) {
+    const double af[4] = {a[k], a[8 * kTp + k], a[k + 4], a[8 * kTp + k + 4]};
+    const double bf[2] = {b[k * kTp], b[(k + 4) * kTp]};
+    dmma(acc, af, bf);
+  }
+}
+
+// In-place inverse of the upper triangular kTb x kTb block T (the identity from row
+// and column kb on): both 32 x 32 halves by a warp each, joined by
+// X12 = -X11 (U12 X22), W (32 rows) between.  Every panel of hplb_getrs waits for one
+// of these, the transposed solve for two: kTb steps with two block barriers and a
+// division each (invert_upper) take about 17 us longer (N = 1000, NB = 64, 32
+// right-hand sides, plain 721 us, now 419; transposed 2.16 ms, now 1.59).
+template <bool UNIT>
+HPLB_DEV void invert_upper_halves(double (*T)[kTp], double (*W)[kTp], int kb) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if(warp == 0) invert_upper32<UNIT>(T, 0, min(32, kb));
+  if(warp == 1 && kb > 32) invert_upper32<UNIT>(T, 32, kb - 32);
+  if(kb <= 32) return;  // U12 is 0
+  const int r = (warp & 1) * 16 + (lane >> 2), c = (warp >> 1) * 8 + 2 * (lane & 3);
+  double    acc[4];
+  __syncthreads();
+  product32(acc, &T[0][32], &T[32][32]);
+#pragma unroll
+  for(int e = 0; e < 4; ++e) W[r + (e >> 1) * 8][c + (e & 1)] = acc[e];
+  __syncthreads();
+  product32(acc, &T[0][0], &W[0][0]);
+#pragma unroll
+  for(int e = 0; e < 4; ++e) T[r + (e >> 1) * 8][32 + c + (e & 1)] = -acc[e];
 }
 
 // Copies of the tile rows r0 .. r0 + kb, columns c0 .. c0 + kc of A into U
@@ -295,7 +365,7 @@ trsm_kernel(const double* __restrict__ A, int64_t ld, int ns, int rows, int nrhs
         S.T[r][c] = v;
     }
     __syncthreads();
-    invert_upper(S.T, kb);
+    invert_upper_halves<LOWER>(S.T, S.U[1], kb);  // U[1]: no tile is on its way to it yet
   }
   double y[4];  // this warp's entries of y (the warps of the first half)
 #pragma unroll
@@ -474,19 +544,19 @@ cudaError_t launch_trsm_form(const double* A, int64_t ld, int ns, int rows, int 
   return cudaGetLastError();
 }
 
-// One launch per group of kNr right-hand sides, each with flags of its own
-// (trsv_flag_ints(ns) per group), zeroed here unless the caller has done so.
+// One launch per kNr right-hand sides.  Upper: their flags zeroed here; lower: flags of
+// their own (trsv_flag_ints(ns) each), zeroed by the caller for many solves at once.
 template <bool LOWER>
 cudaError_t launch_trsm_blocks(const double* A, int64_t ld, int ns, int rows, int nrhs,
                                const double* Y, int64_t ldy, double* X, int64_t ldx, int* flags,
-                               int* status, bool zeroed, cudaStream_t stream, int* launches) {
+                               int* status, cudaStream_t stream, int* launches) {
   if(ns <= 0 || nrhs <= 0) return cudaSuccess;
   const bool vec = reinterpret_cast<uintptr_t>(A) % 16 == 0 && ld % 2 == 0 &&
                    (rows == ns || ns % 2 == 0);
   for(int q = 0; q < nrhs; q += kNr) {
     const int   nr = std::min(kNr, nrhs - q);
     cudaError_t e  = cudaSuccess;
-    if(!zeroed) e = cudaMemsetAsync(flags, 0, trsv_flag_ints(ns) * sizeof(int), stream);
+    if(!LOWER) e = cudaMemsetAsync(flags, 0, trsv_flag_ints(ns) * sizeof(int), stream);
     if(e != cudaSuccess) return e;
     const double* Yq = Y + (size_t)q * (size_t)ldy;
     double*       Xq = X + (size_t)q * (size_t)ldx;
@@ -496,7 +566,7 @@ cudaError_t launch_trsm_blocks(const double* A, int64_t ld, int ns, int rows, in
                                              stream);
     if(e != cudaSuccess) return e;
     ++*launches;
-    if(zeroed) flags += trsv_flag_ints(ns);
+    if(LOWER) flags += trsv_flag_ints(ns);
   }
   return cudaSuccess;
 }
@@ -506,15 +576,15 @@ cudaError_t launch_trsm_blocks(const double* A, int64_t ld, int ns, int rows, in
 cudaError_t launch_trsm_upper(const double* A, int64_t ld, int n, int nrhs, const double* Y,
                               int64_t ldy, double* X, int64_t ldx, int* flags, int* status,
                               cudaStream_t stream, int* launches) {
-  return launch_trsm_blocks<false>(A, ld, n, n, nrhs, Y, ldy, X, ldx, flags, status, false,
-                                   stream, launches);
+  return launch_trsm_blocks<false>(A, ld, n, n, nrhs, Y, ldy, X, ldx, flags, status, stream,
+                                   launches);
 }
 
 cudaError_t launch_trsm_lower(const double* L, int64_t ldl, int ns, int rows, int nrhs, double* X,
-                              int64_t ldx, int* flags, int* status, bool zeroed,
-                              cudaStream_t stream, int* launches) {
-  return launch_trsm_blocks<true>(L, ldl, ns, rows, nrhs, X, ldx, X, ldx, flags, status, zeroed,
-                                  stream, launches);
+                              int64_t ldx, int* flags, int* status, cudaStream_t stream,
+                              int* launches) {
+  return launch_trsm_blocks<true>(L, ldl, ns, rows, nrhs, X, ldx, X, ldx, flags, status, stream,
+                                  launches);
 }
 
 }  // namespace hplb

@@ -168,6 +168,31 @@ def test_getrs_block_edges(hlib, oracle, n, nb, nrhs, trans):
     assert err <= tol, (err, tol)
 
 
+@pytest.mark.parametrize("nrhs", [2, 8, 9, 130])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 31, 32, 33, 48, 63, 64, 65, 97, 161])
+def test_trsm_upper_block_edges(hlib, n, nrhs):
+    """Diagonal blocks of 64 are inverted in two halves of 32, ragged ones to their
+    own size: U X = B with |U X - B| within n + 64 roundings of |U| |U^-1| |U| |X|
+    (a sum of n products, and one of 64 with a block's inverse, whose own error is
+    a sum of 64 more)."""
+    import torch
+
+    rng = np.random.default_rng(100 * n + nrhs)
+    ld = n + n % 2
+    U = np.triu(rng.random((n, n)) - 0.5) + 2.0 * np.eye(n)
+    B = rng.random((n, nrhs)) - 0.5
+    dU = torch.full((n, ld), np.nan, dtype=torch.float64, device="cuda")
+    low = rng.random((n, n))  # what stands below the diagonal is not U's
+    dU[:, :n] = torch.from_numpy(np.ascontiguousarray((U + np.tril(low, -1)).T))
+    dB = torch.from_numpy(np.ascontiguousarray(B.T)).cuda()
+    dX = torch.full_like(dB, np.nan)
+    hlib.trsm_upper(n, nrhs, dU.data_ptr(), ld, dB.data_ptr(), n, dX.data_ptr(), n)
+    X = dX.cpu().numpy().T
+    A = np.abs(U)
+    bound = 2 * (n + 64) * EPS * (A @ np.abs(np.linalg.inv(U)) @ A @ np.abs(X))
+    assert np.all(np.abs(U @ X - B) <= bound)
+
+
 @pytest.mark.parametrize("trans", [0, 1])
 def test_getrs_launches_do_not_grow_with_right_hand_sides(hlib, oracle, trans):
     """Up to 128 right-hand sides a triangular solve is one launch: a chain of row
