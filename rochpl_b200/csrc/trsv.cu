@@ -403,6 +403,7 @@ trsm_kernel(const double* __restrict__ A, int64_t ld, int ns, int rows, int nrhs
   }
 
   // y - sum: the second half's part through shared memory.
+  bool bad = false;  // a value that 0 does not take out of a product
   __syncthreads();
   if(kh != 0)
 #pragma unroll
@@ -414,6 +415,7 @@ trsm_kernel(const double* __restrict__ A, int64_t ld, int ns, int rows, int nrhs
       const int r = rt + g + (e >> 1) * 8, q = 2 * t4 + (e & 1);
       y[e] -= acc[e] + S.X[1][q][r];
       S.X[0][q][r] = y[e];
+      bad |= !isfinite(y[e]);
     }
   }
   if(!solve) {
@@ -425,8 +427,21 @@ trsm_kernel(const double* __restrict__ A, int64_t ld, int ns, int rows, int nrhs
       }
     return;
   }
-  __syncthreads();
-  if(kh == 0) {  // x = D^-1 (y - sum), two chains
+  if(__syncthreads_or(bad)) {
+    // x = D^-1 (y - sum) over D^-1's triangle alone: an infinity or NaN in y reaches
+    // only the rows that depend on it, which the full products below would not keep.
+    if(kh == 0) {
+      for(int e = 0; e < 4; ++e) {
+        const int r = rt + g + (e >> 1) * 8, q = 2 * t4 + (e & 1);
+        if(r >= kb || q >= nq) continue;
+        double x = 0.0;
+        for(int k = LOWER ? 0 : r; k < (LOWER ? r + 1 : kb); ++k)
+          x = fma(LOWER ? S.T[k][r] : S.T[r][k], S.X[0][q][k], x);
+        X[(size_t)(r0 + r) + (size_t)(q0 + q) * (size_t)ldx] = x;
+      }
+      __threadfence();
+    }
+  } else if(kh == 0) {  // x = D^-1 (y - sum), two chains
     double x0[4] = {0.0, 0.0, 0.0, 0.0}, x1[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for(int s = 0; s < kTb; s += 8) {

@@ -193,6 +193,32 @@ def test_trsm_upper_block_edges(hlib, n, nrhs):
     assert np.all(np.abs(U @ X - B) <= bound)
 
 
+@pytest.mark.parametrize("n,row", [(40, 7), (64, 33), (100, 70), (200, 90)])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_trsm_upper_non_finite_rows(hlib, n, row, bad):
+    """An infinity or NaN in y reaches the rows above its own and its own column;
+    the rows below, and the other right-hand sides, are what they are without it, to
+    a sum of n products in another order."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    U = np.triu(rng.random((n, n)) - 0.5) + 2.0 * np.eye(n)
+    B = rng.random((n, 8)) - 0.5
+    dU = torch.from_numpy(np.ascontiguousarray(U.T)).cuda()
+    out = []
+    for y in (None, bad):
+        dX = torch.from_numpy(np.ascontiguousarray(B.T)).cuda()
+        if y is not None:
+            dX[3, row] = y
+        hlib.trsm_upper(n, 8, dU.data_ptr(), n, dX.data_ptr(), n, dX.data_ptr(), n)
+        out.append(dX.cpu().numpy().T)
+    clean, got = out
+    assert not np.any(np.isfinite(got[: row + 1, 3]))
+    got[: row + 1, 3] = clean[: row + 1, 3]
+    bound = 2 * (n + 64) * EPS * (np.abs(np.linalg.inv(U)) @ np.abs(U) @ np.abs(clean))
+    assert np.all(np.abs(got - clean) <= bound)
+
+
 @pytest.mark.parametrize("trans", [0, 1])
 def test_getrs_launches_do_not_grow_with_right_hand_sides(hlib, oracle, trans):
     """Up to 128 right-hand sides a triangular solve is one launch: a chain of row
