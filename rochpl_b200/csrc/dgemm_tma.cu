@@ -35,7 +35,7 @@
 //
 // Every mbarrier wait is bounded: a wait only expires when a copy never lands;
 // the CTA then records the site in the status word and exits.
-#include <cstdlib>
+#include <algorithm>
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -354,15 +354,14 @@ int sm_count() {
 // critical path once the trailing matrix is small) wait less for SMs.
 // Measured at N = 16384 (getrf, NB = 512, B200): 251 ms with four, 208 ms
 // with one, identical bits.
-int tiles_per_cta(long long ntiles) {
-  const long long sms = sm_count();
-  return ntiles >= 1024 * sms ? 8 : (ntiles >= 256 * sms ? 4 : 1);
+int tiles_per_cta(long long ntiles, int sms) {
+  return ntiles >= 1024LL * sms ? 8 : (ntiles >= 256LL * sms ? 4 : 1);
 }
 
 template <class S>
 cudaError_t launch_shape(int m, int n, int k, const double* A, int64_t lda, const double* B,
                          int64_t ldb, double* C, int64_t ldc, int* status, bool accumulate,
-                         cudaStream_t stream, long long tpc) {
+                         cudaStream_t stream, int tpc, unsigned grid) {
   CUtensorMap mA, mB;
   {
     cuuint64_t dims[3]    = {16, (cuuint64_t)k, (cuuint64_t)((m + 15) / 16)};
@@ -394,15 +393,13 @@ cudaError_t launch_shape(int m, int n, int k, const double* A, int64_t lda, cons
     if(e != cudaSuccess) return e;
     attr = true;
   }
-  const int       tiles_m = (m + S::BM - 1) / S::BM, tiles_n = (n + S::BN - 1) / S::BN;
-  const long long grid    = ((long long)tiles_m * tiles_n + tpc - 1) / tpc;
-  if(grid > 0x7fffffff || tpc > 0x7fffffff) return cudaErrorInvalidValue;
+  const int tiles_m = (m + S::BM - 1) / S::BM, tiles_n = (n + S::BN - 1) / S::BN;
   if(accumulate)
-    dgemm_tma_kernel<S, true><<<(unsigned)grid, S::THREADS, S::SMEM_BYTES, stream>>>(
-        mA, mB, m, n, k, C, ldc, tiles_m, tiles_n, (int)tpc, status);
+    dgemm_tma_kernel<S, true><<<grid, S::THREADS, S::SMEM_BYTES, stream>>>(
+        mA, mB, m, n, k, C, ldc, tiles_m, tiles_n, tpc, status);
   else
-    dgemm_tma_kernel<S, false><<<(unsigned)grid, S::THREADS, S::SMEM_BYTES, stream>>>(
-        mA, mB, m, n, k, C, ldc, tiles_m, tiles_n, (int)tpc, status);
+    dgemm_tma_kernel<S, false><<<grid, S::THREADS, S::SMEM_BYTES, stream>>>(
+        mA, mB, m, n, k, C, ldc, tiles_m, tiles_n, tpc, status);
   return cudaGetLastError();
 }
 
@@ -418,20 +415,35 @@ bool dgemm_tma_eligible(int m, int n, int k, const double* A, int64_t lda, const
   return get_encoder();
 }
 
+// Small tiles where the large ones fill at most three quarters of the SMs: the
+// product then takes one large tile's time (k = 256: 33 us) however few there
+// are.  Above that both need as many rounds of the SMs.  Both sum every element
+// in the same order.  A cap holds for the grid of either: two small tiles' CTAs share
+// an SM only once every SM has one, so at most max_ctas SMs are taken.  N = 4096,
+// NB = 256, whose late updates are capped: 10.53 ms with the cap on small tiles,
+// with large ones instead and without a cap there alike.
+void plan_dgemm(int m, int n, int sms, int max_ctas, int* small, long long* tpc,
+                long long* grid) {
+  auto tiles = [&](int bm, int bn) { return (long long)((m + bm - 1) / bm) * ((n + bn - 1) / bn); };
+  long long t = tiles(Large::BM, Large::BN);
+  *small      = t * 4 <= 3LL * sms;
+  if(*small) t = tiles(Small::BM, Small::BN);
+  *tpc = *small ? 1 : tiles_per_cta(t, sms);
+  if(max_ctas > 0) *tpc = std::max(*tpc, (t + max_ctas - 1) / max_ctas);
+  *grid = (t + *tpc - 1) / *tpc;
+}
+
 cudaError_t launch_dgemm_tma(int m, int n, int k, const double* A, int64_t lda, const double* B,
                              int64_t ldb, double* C, int64_t ldc, int* status, bool accumulate,
                              cudaStream_t stream, int max_ctas) {
-  const long long ntiles =
-      (long long)((m + Large::BM - 1) / Large::BM) * ((n + Large::BN - 1) / Large::BN);
-  // Small tiles where the large ones fill at most three quarters of the SMs: the
-  // product then takes one large tile's time (k = 256: 33 us) however few there
-  // are.  Above that both need as many rounds of the SMs.  Both sum every element
-  // in the same order.
-  if(ntiles * 4 <= 3LL * sm_count())
-    return launch_shape<Small>(m, n, k, A, lda, B, ldb, C, ldc, status, accumulate, stream, 1);
-  long long tpc = tiles_per_cta(ntiles);
-  if(max_ctas > 0 && (ntiles + tpc - 1) / tpc > max_ctas) tpc = (ntiles + max_ctas - 1) / max_ctas;
-  return launch_shape<Large>(m, n, k, A, lda, B, ldb, C, ldc, status, accumulate, stream, tpc);
+  int       small;
+  long long tpc, grid;
+  plan_dgemm(m, n, sm_count(), max_ctas, &small, &tpc, &grid);
+  if(grid > 0x7fffffff || tpc > 0x7fffffff) return cudaErrorInvalidValue;
+  return small ? launch_shape<Small>(m, n, k, A, lda, B, ldb, C, ldc, status, accumulate, stream,
+                                     (int)tpc, (unsigned)grid)
+               : launch_shape<Large>(m, n, k, A, lda, B, ldb, C, ldc, status, accumulate, stream,
+                                     (int)tpc, (unsigned)grid);
 }
 
 }  // namespace hplb

@@ -28,6 +28,10 @@ cudaError_t launch_dgemm_set(int m, int n, int k, const double* A, int64_t lda,
                              int* status, cudaStream_t stream);
 bool        dgemm_tma_eligible(int m, int n, int k, const double* A, int64_t lda,
                                const double* B, int64_t ldb);
+// Its tiles for an m x n product on sms SMs: small or large ones, tiles per CTA and
+// the grid, of at most max_ctas CTAs where that is above 0.
+void        plan_dgemm(int m, int n, int sms, int max_ctas, int* small, long long* tpc,
+                       long long* grid);
 cudaError_t launch_dgemm_tma(int m, int n, int k, const double* A, int64_t lda,
                              const double* B, int64_t ldb, double* C, int64_t ldc,
                              int* status, bool accumulate, cudaStream_t stream,
