@@ -484,7 +484,7 @@ static hplb_status residual_common(hplb_ctx* ctx, int n, const double* dA, int64
   if(!lcg && n > 0 && (!dA || ld < n)) return set_err(ctx, HPLB_ERR_ARG, "hplb_residual: bad matrix");
   if(n > 0 && !dX) return set_err(ctx, HPLB_ERR_ARG, "hplb_residual: null solution");
   ENTER(ctx);
-  hplb_status s = grow(ctx, &ctx->d_res, &ctx->res_cap, residual_ws_doubles(std::max(n, 1)));
+  hplb_status s = grow(ctx, &ctx->d_res, &ctx->res_cap, residual_ws_doubles(std::max(n, 1), lcg));
   if(s != HPLB_OK) return s;
   CK(launch_residual(n, dA, ld, lcg, seed, dX, ctx->d_res, ctx->d_out8, ctx->s_upd));
   double o[8];

@@ -134,8 +134,8 @@ cudaError_t launch_gemv_acc(int m, int k, const double* U, int64_t ld, const dou
                             double* z, cudaStream_t stream);
 cudaError_t launch_vsub(int n, const double* y, const double* s, double* r, cudaStream_t stream);
 
-// Residual check.  ws must hold residual_ws_doubles(n) doubles.
-size_t      residual_ws_doubles(int n);
+// Residual check.  ws must hold residual_ws_doubles(n, lcg) doubles.
+size_t      residual_ws_doubles(int n, bool lcg);
 cudaError_t launch_residual(int n, const double* A, int64_t ld, bool lcg, uint64_t seed,
                             const double* X, double* ws, double* out8, cudaStream_t stream);
 
@@ -144,7 +144,7 @@ cudaError_t launch_residual(int n, const double* A, int64_t ld, bool lcg, uint64
 cudaError_t launch_gemv_hpl(int n, const double* A, int64_t ld, bool lcg, uint64_t seed,
                             const double* x, double* y, double* ws, cudaStream_t stream);
 cudaError_t launch_column_hpl(int n, int col, const double* A, int64_t ld, bool lcg,
-                              uint64_t seed, double* out, double* ws, cudaStream_t stream);
+                              uint64_t seed, double* out, cudaStream_t stream);
 
 // Mixed-precision helpers (mixed.cu, sgemm.cu, matgen.cu).
 cudaError_t launch_sgemm(int m, int n, int k, const float* A, int64_t lda, const float* B,

@@ -456,7 +456,7 @@ extern "C" hplb_status hplb_pdgesv_mixed(hplb_ctx* ctx, const hplb_algo* algo,
                2 * nblk * 1024 + 2 * (size_t)nb * nb + nb + 64)) != HPLB_OK ||
      (s = grow(ctx, &ctx->m_vec, &ctx->m_vec_cap,
                Refine::doubles(n, o.restart) + (size_t)n + nb + 16)) != HPLB_OK ||
-     (s = grow(ctx, &ctx->d_res, &ctx->res_cap, residual_ws_doubles(n))) != HPLB_OK)
+     (s = grow(ctx, &ctx->d_res, &ctx->res_cap, residual_ws_doubles(n, !dA))) != HPLB_OK)
     return s;
   M.W = ctx->m_w;
 
@@ -519,7 +519,7 @@ extern "C" hplb_status hplb_pdgesv_mixed(hplb_ctx* ctx, const hplb_algo* algo,
   // ||A||oo, ||b||oo and eps from the residual kernels at x = 0.
   CK(cudaMemsetAsync(dX, 0, (size_t)n * sizeof(double), su));
   CK(launch_residual(n, dA, ld, F.lcg, seed, dX, ctx->d_res, ctx->d_out8, su));
-  CK(launch_column_hpl(n, n, dA, ld, F.lcg, seed, F.b, ctx->d_res, su));
+  CK(launch_column_hpl(n, n, dA, ld, F.lcg, seed, F.b, su));
   ctx->launches += 5;
   double o8[8];
   CK(cudaMemcpyAsync(o8, ctx->d_out8, sizeof o8, cudaMemcpyDeviceToHost, su));

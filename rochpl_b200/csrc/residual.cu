@@ -7,12 +7,16 @@
 // needs no N x N buffer at all.
 //
 // Work split (all reductions in a fixed order, no floating-point atomics):
-//   rows_partial : grid (row blocks, column chunks); per row and chunk the
-//                  partial sums of a_ij x_j and |a_ij|.
+//   rows_partial, rows_cols_partial : grid (row blocks, column chunks); per row and
+//                  chunk the partial sums of a_ij x_j and |a_ij|; the latter, for a
+//                  stored matrix, also per row block and column that of |a_ij|.
 //   rows_final   : per row r_i = b_i - sum, row sum of |a|; per block the
 //                  maxima of |r|, row sums, |b|, |x| and the sum of |x|.
-//   col_sums     : one warp per column: sum_i |a_ij|; per block the max.
+//   col_fold / col_sums : per column sum_i |a_ij| from those sums / regenerated, a
+//                  warp per column; per block the max.
 //   finish       : one block folds the per-block values into the 8 outputs.
+#include <algorithm>
+
 #include "common.cuh"
 #include "internal.h"
 #include "lcg.cuh"
@@ -79,16 +83,17 @@ rows_partial(int n, const double* __restrict__ A, int64_t ld, const double* __re
 // (16 exchanges for 16 columns); the warps' sums meet in shared memory, the
 // CTAs' in part_c (a row of n per 256 rows of A).  Four CTAs per SM, so that one's
 // folding runs under the others' loads: the whole check at N = 16384 takes 480 us
-// (858 with two passes, 725 with 32 columns at a time and two CTAs).  col_sums adds in the same order, so the
-// stored and the regenerated check agree to the last bit.
+// (858 with two passes, 725 with 32 columns at a time and two CTAs).  A has m rows
+// from here on; the chunks' partial row sums are `rows` apart.  col_sums adds in the
+// same order, so the stored and the regenerated check agree to the last bit.
 __global__ void __launch_bounds__(kRowThreads, 4)
-rows_cols_partial(int n, const double* __restrict__ A, int64_t ld, const double* __restrict__ X,
-                  double* part_r, double* part_a, double* part_c) {
+rows_cols_partial(int n, int m, int rows, const double* __restrict__ A, int64_t ld,
+                  const double* __restrict__ X, double* part_r, double* part_a, double* part_c) {
   constexpr int     kW = kRowThreads / 32, kU = 16;
   __shared__ double sc[kW][kPassHalf];
   const int     lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int     i = blockIdx.x * kRowThreads + threadIdx.x;
-  const bool    in = i < n;
+  const bool    in = i < m;
   const int     jb = blockIdx.y * kChunk, je = min(n, jb + kChunk);
   const double* a = A + (in ? i : 0);
   double        acc = 0.0, asum = 0.0;
@@ -128,8 +133,8 @@ rows_cols_partial(int n, const double* __restrict__ A, int64_t ld, const double*
     __syncthreads();
   }
   if(in) {
-    part_r[(size_t)blockIdx.y * n + i] = acc;
-    part_a[(size_t)blockIdx.y * n + i] = asum;
+    part_r[(size_t)blockIdx.y * rows + i] = acc;
+    part_a[(size_t)blockIdx.y * rows + i] = asum;
   }
 }
 
@@ -159,11 +164,11 @@ HPLB_DEV double block_sum(double v, double* sh) {
 
 template <bool LCG>
 __global__ void __launch_bounds__(kRowThreads)
-rows_final(int n, int nch, const double* __restrict__ A, int64_t ld, const double* __restrict__ X,
-           const __grid_constant__ ResTabs T, const double* part_r, const double* part_a,
-           double* blk) {
+rows_final(int n, int row0, int rows, int nch, const double* __restrict__ A, int64_t ld,
+           const double* __restrict__ X, const __grid_constant__ ResTabs T, const double* part_r,
+           const double* part_a, double* blk) {
   __shared__ double sh[32];
-  const int i = blockIdx.x * kRowThreads + threadIdx.x;
+  const int il = blockIdx.x * kRowThreads + threadIdx.x, i = row0 + il;
   double rabs = 0.0, rsum = 0.0, babs = 0.0, xabs = 0.0, xs = 0.0;
   if(i < n) {
     double b;
@@ -173,8 +178,8 @@ rows_final(int n, int nch, const double* __restrict__ A, int64_t ld, const doubl
       b = A[(size_t)i + (size_t)n * ld];
     double acc = 0.0;
     for(int c = 0; c < nch; ++c) {
-      acc += part_r[(size_t)c * n + i];
-      rsum += part_a[(size_t)c * n + i];
+      acc += part_r[(size_t)c * rows + il];
+      rsum += part_a[(size_t)c * rows + il];
     }
     rabs = fabs(b - acc);
     babs = fabs(b);
@@ -196,19 +201,28 @@ rows_final(int n, int nch, const double* __restrict__ A, int64_t ld, const doubl
   }
 }
 
-// The largest column sum of a CTA's 256 columns, from the nrg row groups' sums.
+// Column sums so far (sum; from zero if `first`) and nrg more row groups' of a CTA's
+// 256 columns; the last time, their largest to blkc.
 __global__ void __launch_bounds__(256)
-col_max(int n, int nrg, const double* __restrict__ part_c, double* blkc) {
+col_fold(int n, int nrg, const double* __restrict__ part_c, bool first, bool last, double* sum,
+         double* blkc) {
   __shared__ double sh[32];
   const int j = blockIdx.x * 256 + threadIdx.x;
-  double    s = 0.0;
+  double    s = (first || j >= n) ? 0.0 : sum[j];
   if(j < n)
     for(int g = 0; g < nrg; ++g) s += part_c[(size_t)g * n + j];
+  if(!last) {
+    if(j < n) sum[j] = s;
+    return;
+  }
   const double m = block_max(s, sh);
   if(threadIdx.x == 0) blkc[blockIdx.x] = m;
 }
 
-// Column sums of the regenerated matrix.
+// Column sums of the regenerated matrix, added in the order of rows_cols_partial's
+// folds.  The regenerating check as a whole: N = 1000 0.11 ms, 16384 0.69, 131072 34.2
+// (0.15, 0.73 and 35.3 with lanes that keep sums of their own to the end and four more
+// FP64 steps per entry).
 __global__ void __launch_bounds__(256)
 col_sums(int n, const __grid_constant__ ResTabs T, double* blkc) {
   __shared__ double sh[32];
@@ -285,35 +299,70 @@ ResTabs make_tabs(int n, uint64_t seed) {
 
 }  // namespace
 
-size_t residual_ws_doubles(int n) {
+namespace {
+
+// The stored check's partial column sums take n doubles per 256 rows (n^2 / 256 in
+// all), its partial row sums 2 per row and 2048 columns (n^2 / 1024).  Matrices of
+// more than kOneBand row groups (102400 rows, 84 GB) are read in kBands bands of rows
+// that share the space of one, so that a matrix that fills the GPU needs no more
+// than n^2 / 1024 (N = 131072: 128 MB, one band 671 MB).  Each band's last CTAs run
+// alone for a moment: N = 131072 25.8 -> 26.5 ms, but N = 50000 3.4 -> 5.1, so smaller
+// matrices stay in one.
+constexpr int kOneBand = 400, kBands = 6;
+
+struct Bands {
+  int count, groups;  // bands, and 256-row groups of each but the last
+};
+Bands bands_of(int n) {
+  const int nrb = (n + kRowThreads - 1) / kRowThreads;
+  const int c   = nrb > kOneBand ? kBands : 1;
+  const int g   = (nrb + c - 1) / c;
+  return {(nrb + g - 1) / g, g};
+}
+
+}  // namespace
+
+// Doubles of scratch of the check, and of launch_gemv_hpl, for a stored or a
+// regenerated matrix.
+size_t residual_ws_doubles(int n, bool lcg) {
   const size_t nch = (size_t)(n + kChunk - 1) / kChunk;
   const size_t nrb = (size_t)(n + kRowThreads - 1) / kRowThreads;
   const size_t ncb = (size_t)(n + 7) / 8;
-  const size_t tabs = (sizeof(ResTabs) + 7) / 8;
-  return (2 * nch + nrb) * (size_t)n + 5 * nrb + ncb + tabs + 16;
+  size_t       part = 2 * nch * (size_t)n;
+  if(!lcg) {
+    const Bands b = bands_of(n);
+    part          = std::max(part, 2 * nch * (size_t)b.groups * kRowThreads +
+                                       (size_t)(b.groups + 1) * (size_t)n);
+  }
+  return part + 5 * nrb + ncb + 16;
 }
 
 cudaError_t launch_residual(int n, const double* A, int64_t ld, bool lcg, uint64_t seed,
                             const double* X, double* ws, double* out8, cudaStream_t stream) {
   if(n <= 0) return cudaMemsetAsync(out8, 0, 8 * sizeof(double), stream);
   const int nrb = (n + kRowThreads - 1) / kRowThreads;
+  const int nch = (n + kChunk - 1) / kChunk;
   if(!lcg) {
-    const int nch = (n + kChunk - 1) / kChunk;
-    const int ncb = (n + 255) / 256;
-    double*   part_r = ws;
-    double*   part_a = part_r + (size_t)nch * n;
-    double*   part_c = part_a + (size_t)nch * n;
-    double*   blk    = part_c + (size_t)nrb * n;
-    double*   blkc   = blk + (size_t)nrb * 5;
-    rows_cols_partial<<<dim3(nrb, nch), kRowThreads, 0, stream>>>(n, A, ld, X, part_r, part_a,
-                                                                  part_c);
-    rows_final<false><<<nrb, kRowThreads, 0, stream>>>(n, nch, A, ld, X, ResTabs{}, part_r, part_a,
-                                                       blk);
-    col_max<<<ncb, 256, 0, stream>>>(n, nrb, part_c, blkc);
+    const int    ncb    = (n + 255) / 256;
+    const Bands  b      = bands_of(n);
+    const int    rows   = b.groups * kRowThreads;
+    double*      part_r = ws;
+    double*      part_a = part_r + (size_t)nch * rows;
+    double*      part_c = part_a + (size_t)nch * rows;
+    double*      sum    = part_c + (size_t)b.groups * n;
+    double*      blk    = sum + n;
+    double*      blkc   = blk + (size_t)nrb * 5;
+    for(int k = 0; k < b.count; ++k) {
+      const int g0 = k * b.groups, ng = std::min(b.groups, nrb - g0), row0 = g0 * kRowThreads;
+      rows_cols_partial<<<dim3(ng, nch), kRowThreads, 0, stream>>>(n, n - row0, rows, A + row0, ld, X,
+                                                                   part_r, part_a, part_c);
+      rows_final<false><<<ng, kRowThreads, 0, stream>>>(n, row0, rows, nch, A, ld, X, ResTabs{},
+                                                        part_r, part_a, blk + (size_t)g0 * 5);
+      col_fold<<<ncb, 256, 0, stream>>>(n, ng, part_c, k == 0, k + 1 == b.count, sum, blkc);
+    }
     finish<<<1, 256, 0, stream>>>(n, nrb, ncb, blk, blkc, out8);
     return cudaGetLastError();
   }
-  const int nch = (n + kChunk - 1) / kChunk;
   const int ncb = (n + 7) / 8;
   double* part_r = ws;
   double* part_a = part_r + (size_t)nch * n;
@@ -322,7 +371,7 @@ cudaError_t launch_residual(int n, const double* A, int64_t ld, bool lcg, uint64
   const ResTabs T = make_tabs(n, seed);
   dim3 g1(nrb, nch);
   rows_partial<true><<<g1, kRowThreads, 0, stream>>>(n, A, ld, X, T, part_r, part_a);
-  rows_final<true><<<nrb, kRowThreads, 0, stream>>>(n, nch, A, ld, X, T, part_r, part_a, blk);
+  rows_final<true><<<nrb, kRowThreads, 0, stream>>>(n, 0, n, nch, A, ld, X, T, part_r, part_a, blk);
   col_sums<<<ncb, 256, 0, stream>>>(n, T, blkc);
   finish<<<1, 256, 0, stream>>>(n, nrb, ncb, blk, blkc, out8);
   return cudaGetLastError();
@@ -354,7 +403,7 @@ __global__ void column_of(int n, int col, const double* __restrict__ A, int64_t 
 }  // namespace
 
 // y = A x for the n x n part of [A|b], FP64, from the stored matrix or the LCG.
-// ws: residual_ws_doubles(n) doubles.
+// ws: residual_ws_doubles(n, lcg) doubles.
 cudaError_t launch_gemv_hpl(int n, const double* A, int64_t ld, bool lcg, uint64_t seed,
                             const double* x, double* y, double* ws, cudaStream_t stream) {
   if(n <= 0) return cudaSuccess;
@@ -374,9 +423,8 @@ cudaError_t launch_gemv_hpl(int n, const double* A, int64_t ld, bool lcg, uint64
 
 // out = column col of [A|b] (col = n gives b).
 cudaError_t launch_column_hpl(int n, int col, const double* A, int64_t ld, bool lcg,
-                              uint64_t seed, double* out, double* ws, cudaStream_t stream) {
+                              uint64_t seed, double* out, cudaStream_t stream) {
   if(n <= 0) return cudaSuccess;
-  (void)ws;
   const ResTabs T = make_tabs(n, seed);
   const int nrb = (n + kRowThreads - 1) / kRowThreads;
   if(lcg)
@@ -410,7 +458,7 @@ namespace {
 constexpr int    kNoAllocMaxN = HPLB_NOALLOC_MAX_N;
 constexpr size_t kNoAllocWs   = 2 * ((size_t)(kNoAllocMaxN + kChunk - 1) / kChunk) * kNoAllocMaxN +
                                 5 * ((size_t)(kNoAllocMaxN + kRowThreads - 1) / kRowThreads) +
-                                (size_t)(kNoAllocMaxN + 7) / 8 + (sizeof(ResTabs) + 7) / 8 + 16 + 8;
+                                (size_t)(kNoAllocMaxN + 7) / 8 + 16 + 8;
 
 // Shared by every call on a device; it keeps the last call's contents.  No
 // kernel of the check accumulates into it (every partial sum, per-block value

@@ -261,6 +261,24 @@ def test_residual_pass_edges(hlib, oracle, n):
         assert d1[k] == pytest.approx(o[k], rel=4 * n * EPS, abs=1e-300), k
 
 
+def test_residual_in_bands(hlib):
+    """A stored matrix of more than 102400 rows is read in bands of rows (84 GB: its
+    check against the regenerated one's bits)."""
+    import torch
+
+    n = 102657  # 402 row groups: six bands of 67, the last group of one row
+    ld = n + (-n) % 32
+    if torch.cuda.mem_get_info()[0] < 8 * ld * (n + 1) + (1 << 31):
+        pytest.skip("needs 86 GB of device memory")
+    dA = torch.empty(ld * (n + 1), dtype=torch.float64, device="cuda")
+    hlib.matgen(n, n + 1, 100, dA.data_ptr(), ld)
+    dX = (torch.arange(n, device="cuda") % 7 - 3.0).double() / 5
+    d1 = hlib.residual(n, dA.data_ptr(), ld, dX.data_ptr())
+    assert d1 == hlib.residual_lcg(n, 100, dX.data_ptr())
+    del dA
+    torch.cuda.empty_cache()
+
+
 def test_matgen_long_runs(hlib, oracle):
     """Tall matrices take 64-row runs; the last run of a column is ragged."""
     import torch
