@@ -43,6 +43,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "panel_msgs.h"
 
 namespace hplb {
 
@@ -51,7 +52,6 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarps   = kThreads / 32;
 constexpr int kMaxG    = 16;  // CTAs per cluster at most (non-portable above 8)
-constexpr int kBufs    = 4;   // message buffers, by column
 constexpr int kTri     = 32;  // diagonal block size of the blocked substitution
 constexpr int kMaxOps  = 400;
 constexpr int kMaxNb   = 1024;
@@ -122,18 +122,20 @@ HPLB_DEV bool mbar_try(uint64_t* b, uint32_t parity) {
 }
 // Bounded wait: on expiry the site goes to the status word and every later
 // wait of the CTA returns at once; the kernel then runs to its end on what it
-// has (all positions are range-checked), so no peer is left alone.
-HPLB_DEV void mbar_wait(uint64_t* b, uint32_t parity, volatile int* abort, int* status) {
-  if(mbar_try(b, parity)) return;
+// has (all positions are range-checked), so no peer is left alone, and arms and
+// sends nothing more (panel_msgs.h).  True once the phase has completed.
+HPLB_DEV bool mbar_wait(uint64_t* b, uint32_t parity, volatile int* abort, int* status) {
+  if(mbar_try(b, parity)) return true;
   const unsigned long long t0 = globaltimer();
   while(!mbar_try(b, parity)) {
-    if(*abort) return;
+    if(*abort) return false;
     if(globaltimer() - t0 > kWaitBudgetNs) {
       atomicCAS(status + ST_TIMEOUT, 0, 51);
       *abort = 1;
-      return;
+      return false;
     }
   }
+  return true;
 }
 // 16 bytes into a peer's shared memory, counted by its barrier on arrival.
 HPLB_DEV void push16(uint32_t dst, const double (&v)[2], uint32_t bar) {
@@ -304,7 +306,11 @@ struct Leaf {
   int pos[RPT];   // the rows' positions under the interchanges so far, -1: no row
   T   l[RPT];
 
-  HPLB_DEV uint32_t bytes() const { return G * (uint32_t)(W * sizeof(T) + 16); }
+  HPLB_DEV bool wait(int buf, uint32_t parity) {
+    return mbar_wait(&S.full[buf], parity, &S.abort, P.status);
+  }
+  HPLB_DEV bool expired() const { return S.abort != 0; }
+  HPLB_DEV void arm(int buf) { mbar_expect(&S.full[buf], G * (uint32_t)(W * sizeof(T) + 16)); }
 
   // The block's best candidate of column k1 (register FIRST ? 0 : 1) and its
   // publication by the warp that holds it.  Unless FIRST, the row's columns
@@ -314,6 +320,7 @@ struct Leaf {
   HPLB_DEV void publish(int k1, const T* u) {
     constexpr int I  = FIRST ? 0 : 1;
     const int     d1 = r0 + k1;
+    const bool    sends = may_send(*this);
     Key           key = 0;
     int           bp = -1, bq = 0;
 #pragma unroll
@@ -338,7 +345,7 @@ struct Leaf {
       cp = S.pos[par][lane];
     }
     const int ww = warp_best(ck, cp);
-    if(warp != max(ww, 0)) return;
+    if(warp != max(ww, 0) || !sends) return;
     if(lane == wl) {
 #pragma unroll
       for(int q = 0; q < RPT; ++q)
@@ -403,8 +410,7 @@ struct Leaf {
 #pragma unroll
       for(int q = 0; q < RPT; ++q) odd |= pos[q] >= d && !exponent_safe(x[q][0]);
       odd = __any_sync(0xffffffffu, odd);
-      mbar_wait(&S.full[buf], (kc / kBufs) & 1, &S.abort, P.status);
-      if(threadIdx.x == 0) mbar_expect(&S.full[buf], bytes());
+      const bool arrived = await_column(*this, kc);
       // The winner among the CTAs' candidates; each lane has the reciprocal of
       // its candidate under way while the search runs.
       Key  ck = 0;
@@ -438,7 +444,7 @@ struct Leaf {
         if(pos[q] > d) M.done[k * Mem::pitch + threadIdx.x + q * kThreads] = l[q];
         x[q][1] = fma_(-l[q], u1, x[q][1]);
       }
-      kc += 1;
+      const unsigned kd = kc++;
       if(k + 1 < w) publish<false>(k + 1, u);
       // The other columns, while the candidates travel; the update also moves
       // every column one register down.  Rows that are pivot rows by now, and
@@ -463,6 +469,7 @@ struct Leaf {
       if(warp == kWarps - 1) {
         if(lane >= k && lane < W) S.top[k * kTopPitch + lane] = u[lane - k];
         if(lane == 0) {
+          rearm(*this, kd, arrived);
           S.pv[k] = p - r0;
           if(me == 0) {
             P.ipiv[ca + k] = p;
