@@ -1383,6 +1383,9 @@ struct Builder {
   }
 };
 
+// Launches a cluster of g CTAs; *done stays false where the GPU has no place for one,
+// which is what placeable[g] keeps.  An error is returned and not kept: it may be
+// over by the next call (no memory to load the kernel, say).
 template <typename Kern, typename... Args>
 cudaError_t launch_cluster(Kern kern, int g, size_t smem, signed char* placeable,
                            cudaStream_t stream, bool* done, const Args&... args) {
@@ -1398,28 +1401,24 @@ cudaError_t launch_cluster(Kern kern, int g, size_t smem, signed char* placeable
   at[0].val.clusterDim.z = 1;
   cfg.attrs              = at;
   cfg.numAttrs           = 1;
+  cudaError_t e          = cudaSuccess;
   if(placeable[g] == 0) {  // 0 unknown, 1 yes, -1 no
     int n = 0;
-    if(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-           cudaSuccess ||
-       (g > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-                     cudaSuccess) ||
-       cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
-      cudaGetLastError();
-      placeable[g] = -1;
-    } else {
-      placeable[g] = 1;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if(e == cudaSuccess && g > 8)
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if(e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, kern, &cfg);
+    if(e == cudaSuccess || e == cudaErrorInvalidClusterSize) {
+      placeable[g] = e == cudaSuccess && n >= 1 ? 1 : -1;
+      if(e != cudaSuccess) cudaGetLastError();
+      e = cudaSuccess;
     }
   }
-  if(placeable[g] < 0) return cudaSuccess;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
-  if(e != cudaSuccess) {
-    cudaGetLastError();
-    placeable[g] = -1;
-    return cudaSuccess;
-  }
-  *done = true;
-  return cudaSuccess;
+  if(e == cudaSuccess && placeable[g] < 0) return cudaSuccess;
+  if(e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, kern, args...);
+  *done = e == cudaSuccess;
+  if(!*done) cudaGetLastError();
+  return e;
 }
 
 template <typename T, int W, int RPT>
@@ -1519,8 +1518,8 @@ cudaError_t launch_panel_fused(T* A, int64_t ld, int r0, int c0, int n, int jb, 
     if(last) P.linv = linv;
     bool        did = false;
     cudaError_t e   = launch_rows(P, rows - B.ops[at].off, g, stream, &did);
-    if(e != cudaSuccess) return e;
-    if(!did) return at == 0 ? cudaSuccess : cudaErrorLaunchFailure;
+    if(!did && at == 0) return cudaSuccess;  // (the other path meets a lasting error itself)
+    if(!did) return e != cudaSuccess ? e : cudaErrorLaunchFailure;
     *launches += 1;
     if(!last) {
       const Op& o = B.ops[end - 1];
@@ -1543,14 +1542,15 @@ cudaError_t launch_unit_lower_inverse(const T* L, int64_t ldl, int jb, const T* 
                                       int64_t ldinv, cudaStream_t stream) {
   if(jb <= 0) return cudaSuccess;
   static signed char placeable[kMaxG + 1] = {};
+  cudaError_t e = cudaErrorLaunchFailure;
   for(int g = cluster_for((jb + 31) / 32); g > 0; g /= 2) {
     bool              done = false;
-    const cudaError_t e    = launch_cluster(lower_inverse_kernel<T>, g, kInverseBytes,
-                                            placeable, stream, &done,
-                                            L, ldl, jb, dinv, Linv, ldinv);
-    if(done || e != cudaSuccess) return e;
+    const cudaError_t eg   = launch_cluster(lower_inverse_kernel<T>, g, kInverseBytes, placeable,
+                                            stream, &done, L, ldl, jb, dinv, Linv, ldinv);
+    if(done) return cudaSuccess;
+    if(eg != cudaSuccess) e = eg;
   }
-  return cudaErrorLaunchFailure;
+  return e;
 }
 
 #define HPLB_FUSED_INSTANTIATE(T)                                                               \
