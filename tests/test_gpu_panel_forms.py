@@ -56,6 +56,68 @@ def test_panel_forms_match_the_launch_per_step_panel(hlib, oracle, n, jb, nbmin,
         assert float((a - b).abs().max()) <= 64 * jb * jb * EPS * max(umax, 1.0)
 
 
+def _scaled(n, cols, shifts, seed):
+    """Random entries times powers of two from `shifts`, an exponent per row."""
+    rng = np.random.default_rng(seed)
+    A = rng.random((n, cols)) - 0.5
+    return np.ldexp(A, rng.choice(shifts, size=n)[:, None])
+
+
+@pytest.mark.parametrize("shifts", [
+    [-400, -399, -398], [-402, -401, -400, -399], [498, 499, 500], [499, 500, 501, 502],
+    [-401, 0, 499], [-1050, -1022, -900, 0], [-700, 0, 700]])
+def test_panel_quotients_at_the_exponent_limits(hlib, oracle, shifts):
+    """Multipliers by reciprocal and correction are exact only between 2^-400 and
+    2^500; the rest divide: the bits of the panel that always divides (in global
+    memory: the one across the GPU's registers underflows to +0 whatever the sign)."""
+    import torch
+
+    from rochpl_b200.hpl import Algo
+    from rochpl_b200.lib import LEAF_AUTO, LEAF_GLOBAL
+
+    for n, jb in ((300, 64), (5000, 40)):
+        ld = oracle.default_ld(n)
+        A = torch.zeros((jb, ld), dtype=torch.float64, device="cuda")
+        A[:, :n] = torch.from_numpy(np.ascontiguousarray(_scaled(n, jb, shifts, n).T))
+        out = []
+        for kind in (LEAF_AUTO, LEAF_GLOBAL):
+            B, piv = A.clone(), torch.zeros(jb, dtype=torch.int32, device="cuda")
+            try:
+                hlib.set_leaf(kind)
+                hlib.panel_factor(Algo(jb, 32, 2, 2, 2, 1, 0).c(), n, 0, jb, B.data_ptr(), ld, 0,
+                                  piv.data_ptr())
+            finally:
+                hlib.set_leaf(LEAF_AUTO)
+            out.append((B.view(torch.int64), piv))
+        assert torch.equal(out[0][1], out[1][1])
+        assert torch.equal(out[0][0], out[1][0])
+
+
+@pytest.mark.parametrize("shifts", [[-62, -61, -60, -59], [57, 58, 59, 60], [-61, 0, 59]])
+def test_fp32_panel_quotients_at_the_exponent_limits(hlib, shifts):
+    """The same for the mixed form's FP32 panels (2^-60 to 2^60), by its pivots and
+    solution."""
+    import torch
+
+    from rochpl_b200.hpl import Algo
+    from rochpl_b200.lib import LEAF_AUTO, LEAF_GLOBAL, PREC_FP16X3
+
+    n = 400
+    A = torch.from_numpy(np.ascontiguousarray(_scaled(n, n + 1, shifts, 5).T)).cuda()
+    out = []
+    for kind in (LEAF_AUTO, LEAF_GLOBAL):
+        x = torch.zeros(n, dtype=torch.float64, device="cuda")
+        piv = torch.zeros(n, dtype=torch.int32, device="cuda")
+        try:
+            hlib.set_leaf(kind)
+            hlib.pdgesv_mixed(Algo(64, 32, 2, 2, 2, 1, 0).c(), n, x.data_ptr(), A=A.data_ptr(), ld=n,
+                              precision=PREC_FP16X3, ipiv=piv.data_ptr(), max_outer=1)
+        finally:
+            hlib.set_leaf(LEAF_AUTO)
+        out.append((piv, x.view(torch.int64)))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
 def test_panel_zero_pivot(hlib, oracle):
     from rochpl_b200.lib import LEAF_AUTO
 
