@@ -168,8 +168,7 @@ struct Solve {
       CK(launch_diag_inv(A, ld, j, j, jb, ctx->d_dinv[set], ctx->s_pan));
       ctx->launches += 2;
       CK(launch_unit_lower_inverse(a(j, j), ld, jb, ctx->d_dinv[set], ctx->d_linv[set], jb,
-                                   ctx->s_pan));
-      ctx->launches += 1;
+                                   ctx->s_pan, &ctx->launches));
     }
     CK(cudaEventRecord(e1, ctx->s_pan));
     CK(cudaEventRecord(done, ctx->s_pan));
@@ -572,7 +571,8 @@ hplb_status hplb_panel_update(hplb_ctx* ctx, int n, int j, int jb, const double*
   double* top = dA + (size_t)j + (size_t)c0 * (size_t)ld;
   CK(launch_perm(d_ipiv, j, jb, ctx->d_perm[0], st));
   CK(launch_diag_inv(dL, ldl, 0, 0, jb, ctx->d_dinv[0], st));
-  CK(launch_unit_lower_inverse(dL, ldl, jb, ctx->d_dinv[0], ctx->d_linv[0], jb, st));
+  CK(launch_unit_lower_inverse(dL, ldl, jb, ctx->d_dinv[0], ctx->d_linv[0], jb, st,
+                               &ctx->launches));
   CK(launch_laswp_gather(dA, ld, j, jb, ctx->d_perm[0], ctx->d_w, jb, c0, ncols, st));
   CK(launch_dgemm_set(jb, ncols, jb, ctx->d_linv[0], jb, ctx->d_w, jb, top, ld, ctx->d_status,
                       st));

@@ -88,10 +88,15 @@ template <typename T>
 cudaError_t launch_trsm_node(T* A, int64_t ld, int ia, int jb, int lc, T* dinv_scratch, int c0,
                              int n, cudaStream_t stream, int* launches);
 // Linv (jb x jb, leading dimension ldinv) = L^-1 for the unit-lower L at L
-// (leading dimension ldl) from its 32 x 32 diagonal inverses dinv (panel_fused.cu).
+// (leading dimension ldl) from its 32 x 32 diagonal inverses dinv: by a cluster
+// (panel_fused.cu), or for jb > 512 by substitution on the identity over the GPU
+// (panel.cu).
 template <typename T>
 cudaError_t launch_unit_lower_inverse(const T* L, int64_t ldl, int jb, const T* dinv, T* Linv,
-                                      int64_t ldinv, cudaStream_t stream);
+                                      int64_t ldinv, cudaStream_t stream, int* launches);
+template <typename T>
+cudaError_t launch_unit_lower_inverse_wide(const T* L, int64_t ldl, int jb, const T* dinv, T* Linv,
+                                           int64_t ldinv, cudaStream_t stream, int* launches);
 // X (jb x n) <- L^-1 X for the unit-lower L at L (leading dimension ldl) with
 // its 32 x 32 diagonal inverses dinv (launch_diag_inv), FP64.
 cudaError_t launch_trsm_unit_lower(double* X, int64_t ldx, int jb, const double* L, int64_t ldl,
@@ -161,7 +166,7 @@ cudaError_t launch_pack_u(bool bf16, bool split, int jb, int n, const float* U, 
 // ld); work: 2 jb^2 + jb elements, dinv_work: (jb/32 + 1) * 1024.
 template <typename T>
 cudaError_t launch_upper_inverse(int jb, const T* U, int64_t ld, T* Uinv, T* work, T* dinv_work,
-                                 cudaStream_t st);
+                                 cudaStream_t st, int* launches);
 cudaError_t launch_perm_vec(double* z, int ia, int jb, const int* permU, cudaStream_t st);
 // y -= M x / y = M x with FP32 M (rows x cols, column-major), FP64 x and y
 // (not overlapping).

@@ -463,7 +463,7 @@ cudaError_t launch_pack_u(bool bf16, bool split, int jb, int n, const float* U, 
 
 template <typename T>
 cudaError_t launch_upper_inverse(int jb, const T* U, int64_t ld, T* Uinv, T* work, T* dinv_work,
-                                 cudaStream_t st) {
+                                 cudaStream_t st, int* launches) {
   if(jb <= 0) return cudaSuccess;
   // work: jb*jb (flipped unit lower) + jb*jb (its inverse) + jb (diagonal).
   T* Lf    = work;
@@ -473,15 +473,17 @@ cudaError_t launch_upper_inverse(int jb, const T* U, int64_t ld, T* Uinv, T* wor
   cudaError_t e = cudaGetLastError();
   if(e != cudaSuccess) return e;
   if((e = launch_diag_inv<T>(Lf, jb, 0, 0, jb, dinv_work, st)) != cudaSuccess) return e;
-  if((e = launch_unit_lower_inverse<T>(Lf, jb, jb, dinv_work, Lfinv, jb, st)) != cudaSuccess)
+  if((e = launch_unit_lower_inverse<T>(Lf, jb, jb, dinv_work, Lfinv, jb, st, launches)) !=
+     cudaSuccess)
     return e;
+  *launches += 3;
   upper_flip_out_kernel<T><<<jb, 128, 0, st>>>(jb, Lfinv, d, Uinv);
   return cudaGetLastError();
 }
 template cudaError_t launch_upper_inverse<float>(int, const float*, int64_t, float*, float*,
-                                                 float*, cudaStream_t);
+                                                 float*, cudaStream_t, int*);
 template cudaError_t launch_upper_inverse<double>(int, const double*, int64_t, double*, double*,
-                                                  double*, cudaStream_t);
+                                                  double*, cudaStream_t, int*);
 
 cudaError_t launch_perm_vec(double* z, int ia, int jb, const int* permU, cudaStream_t st) {
   if(jb <= 0) return cudaSuccess;

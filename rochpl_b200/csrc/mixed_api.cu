@@ -121,11 +121,12 @@ struct Mixed {
       if((s = rpanel(j, j, jb, j, jb)) != HPLB_OK) return s;
       CK(launch_perm(ctx->d_ipiv + j, j, jb, perm(p), st));
       CK(launch_diag_inv<float>(W, ldw, j, j, jb, dinv(), st));
-      CK(launch_unit_lower_inverse<float>(w(j, j), ldw, jb, dinv(), linv(p), jb, st));
-      ctx->launches += 3;
+      CK(launch_unit_lower_inverse<float>(w(j, j), ldw, jb, dinv(), linv(p), jb, st,
+                                          &ctx->launches));
+      ctx->launches += 2;
     }
-    CK(launch_upper_inverse(jb, w(j, j), ldw, uinv(p), upper_work(), dinv_piece(), st));
-    ctx->launches += 4;
+    CK(launch_upper_inverse(jb, w(j, j), ldw, uinv(p), upper_work(), dinv_piece(), st,
+                            &ctx->launches));
     CK(cudaEventRecord(p1, st));
     CK(cudaEventRecord(done, st));
     panel_ev.emplace_back(p0, p1);

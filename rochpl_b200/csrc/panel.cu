@@ -1066,6 +1066,14 @@ laswp_gather_kernel(T* A, int64_t ld, int ia, int jb, const int* __restrict__ pe
   }
 }
 
+// Writes the jb x jb identity into X (leading dimension ldx), a CTA per column.
+template <typename T>
+__global__ void identity_kernel(T* X, int64_t ldx, int jb) {
+  const int c = blockIdx.x;
+  for(int r = threadIdx.x; r < jb; r += blockDim.x)
+    X[(size_t)r + (size_t)c * ldx] = r == c ? (T)1 : (T)0;
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -1409,6 +1417,16 @@ cudaError_t launch_trsm_unit_lower(double* X, int64_t ldx, int jb, const double*
 }
 
 template <typename T>
+cudaError_t launch_unit_lower_inverse_wide(const T* L, int64_t ldl, int jb, const T* dinv, T* Linv,
+                                           int64_t ldinv, cudaStream_t stream, int* launches) {
+  identity_kernel<T><<<jb, 128, 0, stream>>>(Linv, ldinv, jb);
+  const cudaError_t e = cudaGetLastError();
+  if(e != cudaSuccess) return e;
+  *launches += 2;
+  return launch_trsm_any<T>(Linv, ldinv, 0, jb, L, ldl, nullptr, dinv, 0, jb, stream);
+}
+
+template <typename T>
 cudaError_t launch_laswp_gather(T* A, int64_t ld, int ia, int jb, const int* permU, T* W,
                                 int64_t ldw, int c0, int n, cudaStream_t stream) {
   if(n <= 0 || jb <= 0) return cudaSuccess;
@@ -1434,6 +1452,8 @@ cudaError_t launch_laswp_gather(T* A, int64_t ld, int ia, int jb, const int* per
                                             int, int, cudaStream_t);                           \
   template cudaError_t launch_trsm_node<T>(T*, int64_t, int, int, int, T*, int, int,            \
                                            cudaStream_t, int*);                                \
+  template cudaError_t launch_unit_lower_inverse_wide<T>(const T*, int64_t, int, const T*, T*, \
+                                                         int64_t, cudaStream_t, int*);         \
   template cudaError_t launch_laswp_gather<T>(T*, int64_t, int, int, const int*, T*, int64_t,  \
                                               int, int, cudaStream_t);
 HPLB_PANEL_INSTANTIATE(double)

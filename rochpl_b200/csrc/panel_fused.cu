@@ -1116,6 +1116,10 @@ HPLB_DEV void tri_tile(const float* A, int64_t lda, int mr, const float* B, int6
 // the identity with L's inverted 32 x 32 diagonal blocks, CP neighbouring columns a
 // warp.
 constexpr int kSubst = 256;
+// The widest inverse that 16 SMs make sooner than substitution over the whole GPU (us
+// in the cluster / over the GPU, FP64: 512 120 / 175, 640 202 / 181, 1024 637 / 426; FP32:
+// 512 133 / 143, 640 224 / 151).
+constexpr int kClusterInverse = 512;
 constexpr size_t kInverseBytes = (size_t)kWarps * 4 * kSubst * sizeof(double);
 static_assert(kInverseBytes >= 2 * kTriStage * sizeof(float), "tri_tile's buffers");
 template <typename T, int CP>
@@ -1183,6 +1187,7 @@ HPLB_DEV void invert_by_substitution(const T* L, int64_t ldl, int jb, const T* d
 // LCG panels of 2048 rows, FP64, |L X - I| / eps in the Frobenius norm and time:
 //   jb = 256  this 274, 34 us;  doubling from 32 on, uncorrected 726, 39 us
 //   jb = 512  this 721, 118 us;  doubling 3744, 77 us;  substitution alone 688, 171 us
+// Beyond kClusterInverse the panel's inverse is substitution over the GPU.
 // (kSubst = 128 takes 51 and 128 us: each product step is a few us of latency.)
 template <typename T>
 HPLB_DEV void lower_inverse(const T* L, int64_t ldl, int jb, const T* dinv, T* X, int64_t ldx,
@@ -1515,7 +1520,7 @@ cudaError_t launch_panel_fused(T* A, int64_t ld, int r0, int c0, int n, int jb, 
     if(!last) ++end;
     P.nops = (int)(end - at);
     std::memcpy(P.ops, B.ops.data() + at, (end - at) * sizeof(Op));
-    if(last) P.linv = linv;
+    if(last && jb <= kClusterInverse) P.linv = linv;
     bool        did = false;
     cudaError_t e   = launch_rows(P, rows - B.ops[at].off, g, stream, &did);
     if(!did && at == 0) return cudaSuccess;  // (the other path meets a lasting error itself)
@@ -1532,22 +1537,36 @@ cudaError_t launch_panel_fused(T* A, int64_t ld, int r0, int c0, int n, int jb, 
     }
     at = end;
   }
-  if(linv && P.linv == nullptr) return cudaErrorLaunchFailure;  // (a panel ends with a leaf)
+  if(linv && jb > kClusterInverse) {
+    cudaError_t e = launch_perm(ipiv + c0, r0, jb, permU, stream);
+    if(e != cudaSuccess) return e;
+    *launches += 1;
+    e = launch_unit_lower_inverse_wide(A + (size_t)r0 + (size_t)c0 * (size_t)ld, ld, jb, dinv, linv,
+                                       jb, stream, launches);
+    if(e != cudaSuccess) return e;
+  } else if(linv && P.linv == nullptr) {
+    return cudaErrorLaunchFailure;  // (a panel ends with a leaf)
+  }
   *done = true;
   return cudaSuccess;
 }
 
 template <typename T>
 cudaError_t launch_unit_lower_inverse(const T* L, int64_t ldl, int jb, const T* dinv, T* Linv,
-                                      int64_t ldinv, cudaStream_t stream) {
+                                      int64_t ldinv, cudaStream_t stream, int* launches) {
   if(jb <= 0) return cudaSuccess;
+  if(jb > kClusterInverse)
+    return launch_unit_lower_inverse_wide(L, ldl, jb, dinv, Linv, ldinv, stream, launches);
   static signed char placeable[kMaxG + 1] = {};
   cudaError_t e = cudaErrorLaunchFailure;
   for(int g = cluster_for((jb + 31) / 32); g > 0; g /= 2) {
     bool              done = false;
     const cudaError_t eg   = launch_cluster(lower_inverse_kernel<T>, g, kInverseBytes, placeable,
                                             stream, &done, L, ldl, jb, dinv, Linv, ldinv);
-    if(done) return cudaSuccess;
+    if(done) {
+      *launches += 1;
+      return cudaSuccess;
+    }
     if(eg != cudaSuccess) e = eg;
   }
   return e;
@@ -1558,7 +1577,7 @@ cudaError_t launch_unit_lower_inverse(const T* L, int64_t ldl, int jb, const T* 
                                              int*, int*, T*, T*, int*, cudaStream_t, int*,      \
                                              bool*);                                            \
   template cudaError_t launch_unit_lower_inverse<T>(const T*, int64_t, int, const T*, T*,       \
-                                                    int64_t, cudaStream_t);
+                                                    int64_t, cudaStream_t, int*);
 HPLB_FUSED_INSTANTIATE(double)
 HPLB_FUSED_INSTANTIATE(float)
 

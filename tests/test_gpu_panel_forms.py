@@ -155,7 +155,7 @@ def _residual(L, X):
 SLACK = 1.25
 
 
-@pytest.mark.parametrize("jb", [33, 64, 65, 128, 200, 255, 257, 400, 511])
+@pytest.mark.parametrize("jb", [33, 64, 65, 128, 200, 255, 257, 400, 512, 513])
 def test_unit_lower_inverse_residual(hlib, oracle, jb):
     """hplb_panel_update on the identity against hplb_laswp_trsm on it."""
     import torch
@@ -172,7 +172,7 @@ def test_unit_lower_inverse_residual(hlib, oracle, jb):
     assert new <= SLACK * sub, (new / EPS, sub / EPS)
 
 
-@pytest.mark.parametrize("jb", [96, 256, 300, 512])
+@pytest.mark.parametrize("jb", [96, 256, 300, 512, 600])
 def test_unit_lower_inverse_residual_fp32(hlib, oracle, jb):
     """The mixed form's FP32 inverse, called by its C++ symbol, against the
     substitution in FP32 on the host."""
@@ -189,11 +189,12 @@ def test_unit_lower_inverse_residual_fp32(hlib, oracle, jb):
     sym = "_ZN4hplb{}IfEE9cudaError{}P11CUstream_st"
     diag = getattr(hlib.L, sym.format("15launch_diag_inv", "PKT_liiiPS2_"))
     diag.argtypes = [P, q, i, i, i, P, P]
-    inv = getattr(hlib.L, sym.format("25launch_unit_lower_inverse", "PKT_liS4_PS2_l"))
-    inv.argtypes = [P, q, i, P, P, q, P]
+    inv = getattr(hlib.L, sym.format("25launch_unit_lower_inverse", "PKT_liS4_PS2_l") + "Pi")
+    inv.argtypes = [P, q, i, P, P, q, P, P]
     torch.cuda.synchronize()
     assert diag(dL.data_ptr(), jb, 0, 0, jb, dinv.data_ptr(), None) == 0
-    assert inv(dL.data_ptr(), jb, jb, dinv.data_ptr(), X.data_ptr(), jb, None) == 0
+    assert inv(dL.data_ptr(), jb, jb, dinv.data_ptr(), X.data_ptr(), jb, None,
+               ctypes.byref(i(0))) == 0
     torch.cuda.synchronize()
     ref = np.eye(jb, dtype=np.float32)
     for b in range(0, jb, 32):  # 32 rows by their block's inverse, as on the GPU
