@@ -415,10 +415,11 @@ bool dgemm_tma_eligible(int m, int n, int k, const double* A, int64_t lda, const
   return get_encoder();
 }
 
-// Small tiles where the large ones fill at most three quarters of the SMs: the
-// product then takes one large tile's time (k = 256: 33 us) however few there
-// are.  Above that both need as many rounds of the SMs.  Both sum every element
-// in the same order.  A cap holds for the grid of either: two small tiles' CTAs share
+// Small tiles where the large ones fill at most two thirds of the SMs: the product
+// then takes one large tile's time (k = 256: 33 us) however few there are.  Above
+// that the small ones need as many rounds of the SMs (whole calls, k = 256, 148 SMs,
+// large -> small: 72 tiles 77 -> 56 us, 84 73 -> 70, 96 73 -> 70, 105 70 -> 74,
+// 110 71 -> 75).  Both sum every element in the same order.  A cap holds for the grid of either: two small tiles' CTAs share
 // an SM only once every SM has one, so at most max_ctas SMs are taken.  N = 4096,
 // NB = 256, whose late updates are capped: 10.53 ms with the cap on small tiles,
 // with large ones instead and without a cap there alike.
@@ -426,7 +427,7 @@ void plan_dgemm(int m, int n, int sms, int max_ctas, int* small, long long* tpc,
                 long long* grid) {
   auto tiles = [&](int bm, int bn) { return (long long)((m + bm - 1) / bm) * ((n + bn - 1) / bn); };
   long long t = tiles(Large::BM, Large::BN);
-  *small      = t * 4 <= 3LL * sms;
+  *small      = t * 3 <= 2LL * sms;
   if(*small) t = tiles(Small::BM, Small::BN);
   *tpc = *small ? 1 : tiles_per_cta(t, sms);
   if(max_ctas > 0) *tpc = std::max(*tpc, (t + max_ctas - 1) / max_ctas);
