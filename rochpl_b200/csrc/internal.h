@@ -88,9 +88,9 @@ template <typename T>
 cudaError_t launch_trsm_node(T* A, int64_t ld, int ia, int jb, int lc, T* dinv_scratch, int c0,
                              int n, cudaStream_t stream, int* launches);
 // Linv (jb x jb, leading dimension ldinv) = L^-1 for the unit-lower L at L
-// (leading dimension ldl) from its 32 x 32 diagonal inverses dinv: by a cluster
-// (panel_fused.cu), or for jb > 512 by substitution on the identity over the GPU
-// (panel.cu).
+// (leading dimension ldl) from its 32 x 32 diagonal inverses dinv, by substitution on
+// the identity: up to 512 columns as the panel does (panel_fused.cu), beyond over the
+// whole GPU (panel.cu).  Both give the same bits.
 template <typename T>
 cudaError_t launch_unit_lower_inverse(const T* L, int64_t ldl, int jb, const T* dinv, T* Linv,
                                       int64_t ldinv, cudaStream_t stream, int* launches);

@@ -972,167 +972,30 @@ HPLB_DEV void gemm_tiles(int m, int n, int k, const float* A, int64_t lda, const
     }
 }
 
-// FP64: a 16 x 32 tile of the products below for a warp, straight from L2 by
-// DMMA: acc = sum over k in [k0, k1) of A(r, k) B(k, c), A column-major (of a
-// strictly lower A, `step` 2, the entries k < at + r), B by its two strides; then
-// out(r, c), at out[r sr + c sc], is acc (step 0), -acc (1), out + B(at + r, c) + acc
-// (2) or out - acc (3).  What stands there already is loaded before the sum.
-HPLB_DEV void tri_warp(const double* A, int64_t lda, int mr, const double* B, int64_t sbk,
-                       int64_t sbn, int nc, int k0, int k1, int step, int at, double* out,
-                       int64_t sr, int64_t sc) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
-  double    acc[4][4], old[4][4];
-#pragma unroll
-  for(int j = 0; j < 4; ++j)
-#pragma unroll
-    for(int r = 0; r < 4; ++r) {
-      const int  rr = g + (r >> 1) * 8, cc = j * 8 + 2 * t4 + (r & 1);
-      const bool in = rr < mr && cc < nc;
-      acc[j][r]     = (in && step == 2) ? __ldcg(B + (size_t)(at + rr) * sbk + (size_t)cc * sbn) : 0.0;
-      old[j][r]     = (in && step >= 2) ? __ldcg(out + (size_t)rr * sr + (size_t)cc * sc) : 0.0;
-    }
-#pragma unroll
-  for(int j = 0; j < 4; ++j)
-#pragma unroll
-    for(int r = 0; r < 4; ++r) {
-      old[j][r] += acc[j][r];
-      acc[j][r] = 0.0;
-    }
-#pragma unroll 4
-  for(int k = k0; k < k1; k += 8) {
-    double a[4], b[4][2];
-#pragma unroll
-    for(int r = 0; r < 4; ++r) {
-      const int rr = g + (r & 1) * 8, kk = k + t4 + (r >> 1) * 4;
-      a[r] = (rr < mr && kk < k1 && (step != 2 || kk < at + rr)) ? __ldcg(A + (size_t)rr + (size_t)kk * lda) : 0.0;
-    }
-#pragma unroll
-    for(int j = 0; j < 4; ++j)
-#pragma unroll
-      for(int h = 0; h < 2; ++h) {
-        const int cc = j * 8 + g, kk = k + t4 + h * 4;
-        b[j][h] = (cc < nc && kk < k1) ? __ldcg(B + (size_t)kk * sbk + (size_t)cc * sbn) : 0.0;
-      }
-#pragma unroll
-    for(int j = 0; j < 4; ++j) dmma(acc[j], a, b[j]);
-  }
-#pragma unroll
-  for(int j = 0; j < 4; ++j)
-#pragma unroll
-    for(int r = 0; r < 4; ++r) {
-      const int rr = g + (r >> 1) * 8, cc = j * 8 + 2 * t4 + (r & 1);
-      if(rr < mr && cc < nc)
-        out[(size_t)rr * sr + (size_t)cc * sc] =
-            (step & 1) ? old[j][r] - acc[j][r] : old[j][r] + acc[j][r];
-    }
-}
-
-// FP32: the same for a 64 x 64 tile by a CTA.  B by its two strides (one of them
-// 1); k-slices of 32 through two cp.async buffers (the triangular factor, B in
-// step 0 and A in the others, with its tile at row or column `at`: what stands
-// above its diagonal blocks, in step 2 above the strict triangle, is not its own
-// and counts as 0).
-constexpr int kTriTile = 64, kTriK = 32, kTriPa = kTriTile + 4, kTriPb = kTriK + 4;
-constexpr int kTriStage = kTriK * kTriPa + kTriTile * kTriPb;  // elements of a buffer
-
-HPLB_DEV void tri_step(float (&acc)[16], const float* as, const float* bs) {
-  const int ty = threadIdx.x % 16, tx = threadIdx.x / 16;
-#pragma unroll 2
-  for(int k = 0; k < kTriK; k += 4) {
-    float4 b[4];
-#pragma unroll
-    for(int j = 0; j < 4; ++j)
-      b[j] = *reinterpret_cast<const float4*>(bs + (tx * 4 + j) * kTriPb + k);
-#pragma unroll
-    for(int q = 0; q < 4; ++q) {
-      const float4 a = *reinterpret_cast<const float4*>(as + (k + q) * kTriPa + ty * 4);
-#pragma unroll
-      for(int j = 0; j < 4; ++j) {
-        const float bv = q == 0 ? b[j].x : q == 1 ? b[j].y : q == 2 ? b[j].z : b[j].w;
-        acc[4 * j]     = fmaf(a.x, bv, acc[4 * j]);
-        acc[4 * j + 1] = fmaf(a.y, bv, acc[4 * j + 1]);
-        acc[4 * j + 2] = fmaf(a.z, bv, acc[4 * j + 2]);
-        acc[4 * j + 3] = fmaf(a.w, bv, acc[4 * j + 3]);
-      }
-    }
-  }
-}
-HPLB_DEV void tri_tile(const float* A, int64_t lda, int mr, const float* B, int64_t sbk, int64_t sbn,
-                       int nc, int k0, int k1, int step, int at, float* out, int64_t sr, int64_t sc,
-                       float* sm) {
-  auto load = [&](int kb, float* st) {
-#pragma unroll
-    for(int h = 0; h < kTriTile * kTriK / kThreads; ++h) {
-      const int  e = threadIdx.x + h * kThreads, r = e % kTriTile, k = e / kTriTile;
-      const int  end = step == 0 ? k1 : step == 2 ? at + r : at + r / kTri * kTri + kTri;
-      const bool in  = r < mr && kb + k < min(k1, end);
-      cp_async1(s_addr(st + k * kTriPa + r), in ? A + (size_t)r + (size_t)(kb + k) * lda : A, in);
-    }
-    float* sb = st + kTriK * kTriPa;
-#pragma unroll
-    for(int h = 0; h < kTriTile * kTriK / kThreads; ++h) {
-      const int  e = threadIdx.x + h * kThreads;
-      const int  k = sbk == 1 ? e % kTriK : e / kTriTile, c = sbk == 1 ? e / kTriK : e % kTriTile;
-      const bool in = c < nc && kb + k < k1 && (step != 0 || kb + k >= at + c / kTri * kTri);
-      cp_async1(s_addr(sb + c * kTriPb + k), in ? B + (size_t)(kb + k) * sbk + (size_t)c * sbn : B,
-                in);
-    }
-    cp_commit();
-  };
-  load(k0, sm);
-  float acc[16], old[16];
-#pragma unroll
-  for(int e = 0; e < 16; ++e) {
-    const int  r = threadIdx.x % 16 * 4 + (e & 3), c = threadIdx.x / 16 * 4 + (e >> 2);
-    const bool in = r < mr && c < nc;
-    acc[e]        = (in && step == 2) ? __ldcg(B + (size_t)(at + r) * sbk + (size_t)c * sbn) : 0.f;
-    old[e]        = (in && step >= 2) ? __ldcg(out + (size_t)r * sr + (size_t)c * sc) : 0.f;
-  }
-#pragma unroll
-  for(int e = 0; e < 16; ++e) {
-    old[e] += acc[e];
-    acc[e] = 0.f;
-  }
-  int buf = 0;
-  for(int kb = k0; kb < k1; kb += kTriK, buf ^= 1) {
-    if(kb + kTriK < k1)
-      load(kb + kTriK, sm + (buf ^ 1) * kTriStage);
-    else
-      cp_commit();
-    cp_wait<1>();
-    __syncthreads();
-    tri_step(acc, sm + buf * kTriStage, sm + buf * kTriStage + kTriK * kTriPa);
-    __syncthreads();
-  }
-#pragma unroll
-  for(int e = 0; e < 16; ++e) {
-    const int r = threadIdx.x % 16 * 4 + (e & 3), c = threadIdx.x / 16 * 4 + (e >> 2);
-    if(r < mr && c < nc)
-      out[(size_t)r * sr + (size_t)c * sc] = (step & 1) ? old[e] - acc[e] : old[e] + acc[e];
-  }
-}
-
-// Inverses of the kSubst x kSubst diagonal blocks of L into X by substitution on
-// the identity with L's inverted 32 x 32 diagonal blocks, CP neighbouring columns a
-// warp.
-constexpr int kSubst = 256;
-// The widest inverse that 16 SMs make sooner than substitution over the whole GPU (us
-// in the cluster / over the GPU, FP64: 512 120 / 175, 640 202 / 181, 1024 637 / 426; FP32:
-// 512 133 / 143, 640 224 / 151).
-constexpr int kClusterInverse = 512;
-constexpr size_t kInverseBytes = (size_t)kWarps * 4 * kSubst * sizeof(double);
-static_assert(kInverseBytes >= 2 * kTriStage * sizeof(float), "tri_tile's buffers");
+// X (jb x jb, leading dimension ldx) = L^-1 for the unit-lower L at L, from its
+// inverted 32 x 32 diagonal blocks (dinv): substitution on the identity, CP
+// neighbouring columns a warp, x in shared memory, one 32-row block after the other.
+// Bound by the loads of L from L2, a batch of 16 columns on its way while the one
+// before is used (FP64 / FP32 at jb = 256 37 / 34 us, 512 132 / 124; 171 / 188 without).
+// Doubling ([A 0; B C]^-1 = [A^-1 0; -C^-1 (B A^-1) C^-1]) has a shorter chain and
+// takes 77 us at 512, but multiplies the rounding of its products by C once more:
+// |L X - I| is then 1.5 times substitution's at jb = 128, 2.7 at 256, 5.4 at 512.
+constexpr int kClusterInverse = 512;  // the widest made here (see launch_unit_lower_inverse)
+constexpr size_t kInverseBytes = (size_t)kWarps * 4 * kClusterInverse * sizeof(double);
 template <typename T, int CP>
-HPLB_DEV void invert_by_substitution(const T* L, int64_t ldl, int jb, const T* dinv, T* X,
-                                     int64_t ldx, int gw, int nw, T* sm) {
+HPLB_DEV void lower_inverse_cols(const T* L, int64_t ldl, int jb, const T* dinv, T* X, int64_t ldx,
+                                 int gw, int nw, T* sm) {
   const int lane = threadIdx.x & 31;
-  T*        x    = sm + (size_t)(threadIdx.x >> 5) * CP * kSubst;  // by column, rows of the block
+  T*        x    = sm + (size_t)(threadIdx.x >> 5) * CP * kClusterInverse;  // by column
   for(int c = gw * CP; c < jb; c += nw * CP) {
-    const int base = c / kSubst * kSubst, m = min(kSubst, jb - base);
-    const int first = (c - base) / kTri * kTri;  // the columns' own 32 rows
-    for(int row0 = first; row0 < m; row0 += kTri) {
-      const int r = base + row0 + lane;
-      const T*  d = dinv + (size_t)(base + row0) / kTri * kTri * kTri;
+    const int first = c / kTri * kTri;  // the columns' own 32 rows; zeros above
+#pragma unroll
+    for(int q = 0; q < CP; ++q)
+      if(c + q < jb)
+        for(int r = lane; r < first; r += 32) X[(size_t)r + (size_t)(c + q) * (size_t)ldx] = (T)0;
+    for(int row0 = first; row0 < jb; row0 += kTri) {
+      const int r = row0 + lane;
+      const T*  d = dinv + (size_t)row0 * kTri;
       T         v[CP];
       if(row0 == first) {
 #pragma unroll
@@ -1140,33 +1003,40 @@ HPLB_DEV void invert_by_substitution(const T* L, int64_t ldl, int jb, const T* d
       } else {
         T dv[kTri];
 #pragma unroll
-        for(int k = 0; k < kTri; ++k) dv[k] = row0 + k < m ? __ldcg(d + k * kTri + lane) : (T)0;
+        for(int k = 0; k < kTri; ++k) dv[k] = row0 + k < jb ? __ldcg(d + k * kTri + lane) : (T)0;
 #pragma unroll
         for(int q = 0; q < CP; ++q) v[q] = (T)0;
-        for(int k = first; k < row0; k += 16) {
-          T lv[16];
+        const T* l = L + min(r, jb - 1);
+        T        lv[2][16];
 #pragma unroll
-          for(int t = 0; t < 16; ++t)
-            lv[t] = r < jb ? __ldcg(L + (size_t)r + (size_t)(base + k + t) * (size_t)ldl) : (T)0;
+        for(int t = 0; t < 16; ++t) lv[0][t] = __ldcg(l + (size_t)(first + t) * (size_t)ldl);
+        for(int k = first; k < row0; k += 32) {
 #pragma unroll
-          for(int t = 0; t < 16; ++t)
+          for(int h = 0; h < 2; ++h) {
+            const int kn = min(k + 16 * (h + 1), row0 - 16);
 #pragma unroll
-            for(int q = 0; q < CP; ++q) v[q] = fma_(-lv[t], x[q * kSubst + k + t], v[q]);
+            for(int t = 0; t < 16; ++t) lv[h ^ 1][t] = __ldcg(l + (size_t)(kn + t) * (size_t)ldl);
+#pragma unroll
+            for(int t = 0; t < 16; ++t)
+#pragma unroll
+              for(int q = 0; q < CP; ++q)
+                v[q] = fma_(-lv[h][t], x[q * kClusterInverse + k + 16 * h + t], v[q]);
+          }
         }
 #pragma unroll
-        for(int q = 0; q < CP; ++q) x[q * kSubst + row0 + lane] = r < jb ? v[q] : (T)0;
+        for(int q = 0; q < CP; ++q) x[q * kClusterInverse + r] = r < jb ? v[q] : (T)0;
         __syncwarp();
 #pragma unroll
         for(int q = 0; q < CP; ++q) v[q] = (T)0;
 #pragma unroll
         for(int k = 0; k < kTri; ++k)
 #pragma unroll
-          for(int q = 0; q < CP; ++q) v[q] = fma_(dv[k], x[q * kSubst + row0 + k], v[q]);
+          for(int q = 0; q < CP; ++q) v[q] = fma_(dv[k], x[q * kClusterInverse + row0 + k], v[q]);
         __syncwarp();
       }
 #pragma unroll
       for(int q = 0; q < CP; ++q) {
-        x[q * kSubst + row0 + lane] = v[q];
+        x[q * kClusterInverse + r] = v[q];
         if(r < jb && c + q < jb) X[(size_t)r + (size_t)(c + q) * (size_t)ldx] = v[q];
       }
       __syncwarp();
@@ -1174,79 +1044,24 @@ HPLB_DEV void invert_by_substitution(const T* L, int64_t ldl, int jb, const T* d
   }
 }
 
-// X (jb x jb, leading dimension ldx) = L^-1 for the unit-lower L at L, from its
-// inverted 32 x 32 diagonal blocks: blocks of kSubst columns by substitution, wider
-// ones by doubling: for neighbouring blocks of s columns, [A 0; B C]^-1 =
-// [A^-1 0; X21 C^-1] with X21 = -C^-1 T, T = B A^-1, each product a tile per warp
-// (FP64) or CTA (FP32, whose FFMA loop wants its operands in shared memory).  T
-// waits, transposed, in X's block above the diagonal.
-//
-// The rounding of T and of the product meets C again in L X - I, the residual that
-// U12 = L11^-1 A12 sees, and grows with |C| |C^-1|; substitution has no such growth.
-// Hence X21 -= C^-1 (T + C X21), which brings the residual back to substitution's.
-// LCG panels of 2048 rows, FP64, |L X - I| / eps in the Frobenius norm and time:
-//   jb = 256  this 274, 34 us;  doubling from 32 on, uncorrected 726, 39 us
-//   jb = 512  this 721, 118 us;  doubling 3744, 77 us;  substitution alone 688, 171 us
-// Beyond kClusterInverse the panel's inverse is substitution over the GPU.
-// (kSubst = 128 takes 51 and 128 us: each product step is a few us of latency.)
 template <typename T>
 HPLB_DEV void lower_inverse(const T* L, int64_t ldl, int jb, const T* dinv, T* X, int64_t ldx,
                             unsigned G, unsigned me, T* sm) {
   const int gw = (int)me + (int)G * (int)(threadIdx.x >> 5), nw = (int)G * kWarps;
-  const int lane = threadIdx.x & 31;
   // Columns per warp: as few passes as four at once allow.
   if(jb <= nw)
-    invert_by_substitution<T, 1>(L, ldl, jb, dinv, X, ldx, gw, nw, sm);
+    lower_inverse_cols<T, 1>(L, ldl, jb, dinv, X, ldx, gw, nw, sm);
   else if(jb <= 2 * nw)
-    invert_by_substitution<T, 2>(L, ldl, jb, dinv, X, ldx, gw, nw, sm);
+    lower_inverse_cols<T, 2>(L, ldl, jb, dinv, X, ldx, gw, nw, sm);
   else
-    invert_by_substitution<T, 4>(L, ldl, jb, dinv, X, ldx, gw, nw, sm);
-  for(int s = kSubst; s < jb; s *= 2) {
-    constexpr bool wide = sizeof(T) == 4;
-    constexpr int  TR = wide ? kTriTile : 16, TC = wide ? kTriTile : 32;
-    const int      tr = (s + TR - 1) / TR, tc = (s + TC - 1) / TC;
-    const int      units = (jb + 2 * s - 1) / (2 * s) * tr * tc;
-    // Step 0: T = B A^-1.  1: X21 = -C^-1 T.  2: T += C X21 (X21 itself and the
-    // strict triangle of L's C).  3: X21 -= C^-1 T.
-    for(int step = 0; step < 4; ++step) {
-      cluster_sync();
-      for(int e = wide ? (int)me : gw; e < units; e += wide ? (int)G : nw) {
-        const int base = e / (tr * tc) * 2 * s, r = e / tc % tr * TR, c = e % tc * TC;
-        const int s2 = min(s, jb - base - s), mr = s2 - r;
-        if(mr <= 0) continue;
-        const bool to_t = (step & 1) == 0;
-        const int  low  = base + s;                           // C's first row
-        T*         bt   = X + (size_t)base + (size_t)low * ldx;  // T^t
-        const T* A = step == 0   ? L + (size_t)(low + r) + (size_t)base * ldl
-                     : step == 2 ? L + (size_t)(low + r) + (size_t)low * ldl
-                                 : X + (size_t)(low + r) + (size_t)low * ldx;
-        const T* B = step == 0   ? X + (size_t)base + (size_t)(base + c) * ldx
-                     : step == 2 ? X + (size_t)low + (size_t)(base + c) * ldx
-                                 : bt + c;
-        T* out = to_t ? bt + (size_t)c + (size_t)r * ldx
-                      : X + (size_t)(low + r) + (size_t)(base + c) * ldx;
-        const int64_t lda = to_t ? ldl : ldx, sbk = to_t ? 1 : ldx, sbn = to_t ? ldx : 1;
-        // The triangular factor's columns from the tile's on, rows up to its last.
-        const int k0 = step == 0 ? c / kTri * kTri : 0;
-        const int k1 = step == 0 ? s : min(s2, (r + TR + kTri - 1) / kTri * kTri);
-        const int at = step == 0 ? c : r;
-        if constexpr(wide)
-          tri_tile(A, lda, mr, B, sbk, sbn, s - c, k0, k1, step, at, out, sbn, sbk, sm);
-        else
-          tri_warp(A, lda, mr, B, sbk, sbn, s - c, k0, k1, step, at, out, sbn, sbk);
-      }
-    }
-  }
-  cluster_sync();
-  for(int c = gw; c < jb; c += nw)
-    for(int r = lane; r < c / kTri * kTri; r += 32) X[(size_t)r + (size_t)c * ldx] = (T)0;
+    lower_inverse_cols<T, 4>(L, ldl, jb, dinv, X, ldx, gw, nw, sm);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 lower_inverse_kernel(const T* L, int64_t ldl, int jb, const T* dinv, T* X, int64_t ldx) {
   extern __shared__ __align__(128) unsigned char dyn[];
-  lower_inverse<T>(L, ldl, jb, dinv, X, ldx, cta_count(), cta_rank(), reinterpret_cast<T*>(dyn));
+  lower_inverse<T>(L, ldl, jb, dinv, X, ldx, gridDim.x, blockIdx.x, reinterpret_cast<T*>(dyn));
 }
 
 constexpr size_t at_least(size_t a, size_t b) { return a > b ? a : b; }
@@ -1551,25 +1366,27 @@ cudaError_t launch_panel_fused(T* A, int64_t ld, int r0, int c0, int n, int jb, 
   return cudaSuccess;
 }
 
+// As in the panel up to kClusterInverse columns, with a CTA per 8 columns over the GPU
+// beyond, where 16 SMs are too few (us at 512 columns, 16 CTAs / the GPU: FP64 132 /
+// 175, FP32 124 / 143; the GPU at 640 181 and 151).
 template <typename T>
 cudaError_t launch_unit_lower_inverse(const T* L, int64_t ldl, int jb, const T* dinv, T* Linv,
                                       int64_t ldinv, cudaStream_t stream, int* launches) {
   if(jb <= 0) return cudaSuccess;
   if(jb > kClusterInverse)
     return launch_unit_lower_inverse_wide(L, ldl, jb, dinv, Linv, ldinv, stream, launches);
-  static signed char placeable[kMaxG + 1] = {};
-  cudaError_t e = cudaErrorLaunchFailure;
-  for(int g = cluster_for((jb + 31) / 32); g > 0; g /= 2) {
-    bool              done = false;
-    const cudaError_t eg   = launch_cluster(lower_inverse_kernel<T>, g, kInverseBytes, placeable,
-                                            stream, &done, L, ldl, jb, dinv, Linv, ldinv);
-    if(done) {
-      *launches += 1;
-      return cudaSuccess;
-    }
-    if(eg != cudaSuccess) e = eg;
-  }
-  return e;
+  static bool attr = false;
+  cudaError_t e    = cudaSuccess;
+  if(!attr)
+    e = cudaFuncSetAttribute(lower_inverse_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kInverseBytes);
+  if(e != cudaSuccess) return e;
+  attr = true;
+  // As many warps as a panel's cluster has; they do not wait for each other.
+  lower_inverse_kernel<T><<<cluster_for((jb + 31) / 32), kThreads, kInverseBytes, stream>>>(
+      L, ldl, jb, dinv, Linv, ldinv);
+  *launches += 1;
+  return cudaGetLastError();
 }
 
 #define HPLB_FUSED_INSTANTIATE(T)                                                               \
