@@ -190,7 +190,8 @@ trsv_kernel(const double* __restrict__ A, int64_t ld, int n, const double* __res
 // tile is staged by asynchronous copies (two buffers) beside the published block
 // x_j, and the CTA's product is a DMMA m16n8k8 per warp and 8 columns (4 row
 // tiles, the 64 columns in two halves).  Then x = D^-1 (y - sum) with the
-// diagonal block inverted while the first tile lands.
+// diagonal block (of a lower one its halves of 32) inverted while the first tile
+// lands.
 //
 // Bound by the chain of row blocks: flag, x_j, one tile product, D^-1 product,
 // store, flag.  Eight right-hand sides per CTA (four CTAs share a tile through
@@ -233,9 +234,12 @@ HPLB_DEV void dmma(double (&d)[4], const double (&a)[4], const double (&b)[2]) {
       : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
-// In-place inverse by a warp of the upper triangular w x w block at (o, o) of T
-// (the identity from w on), a column per lane, from the last row up: a step's row is
-// final in s[31] and the rows above it move one register up.
+// In-place inverse X by a warp of the upper triangular w x w block at (o, o) of T (the
+// identity from w on), a row of X per lane, column by column: a step's column is final
+// in s[0]; the columns after it move one register down.  So X T = I is solved for: with
+// T X = I, a column per lane, U x - y is smaller but the solution of A x = b is worse
+// (|A x - b| 1.3 times as large at n = 64); of L, whose transpose T is, it solves for
+// the columns of L^-1.
 template <bool UNIT>
 HPLB_DEV void invert_upper32(double (*T)[kTp], int o, int w) {
   constexpr int kW = 32;
@@ -243,24 +247,25 @@ HPLB_DEV void invert_upper32(double (*T)[kTp], int o, int w) {
   const double  d = UNIT ? 1.0 : 1.0 / T[o + lane][o + lane];
   double        s[kW];
 #pragma unroll
-  for(int i = 0; i < kW; ++i) s[kW - 1 - i] = w - 1 - i == lane ? 1.0 : 0.0;
-  int k = w - 1;
+  for(int i = 0; i < kW; ++i) s[i] = i == lane ? 1.0 : 0.0;
+  int k = 0;
 #pragma unroll
-  for(int half = 0; half < 2; ++half) {  // the second with half of the rows left
+  for(int half = 0; half < 2; ++half) {  // the second with half of the columns left
 #pragma unroll 1
-    for(; k >= (half == 0 ? kW / 2 : 0); --k) {
+    for(; k < w && (half == 1 || k < kW / 2); ++k) {
       const double dk = UNIT ? 1.0 : __shfl_sync(0xffffffffu, d, k);
-      const double x  = lane >= k ? s[kW - 1] * dk : 0.0;
+      const double x  = lane <= k ? s[0] * dk : 0.0;
 #pragma unroll
       for(int h = 0; h < (half == 0 ? kW : kW / 2); h += kW / 4) {
         double u[kW / 4];
 #pragma unroll
-        for(int i = 0; i < kW / 4; ++i) u[i] = h + i < k ? T[o + k - 1 - h - i][o + k] : 0.0;
+        for(int t = 0; t < kW / 4; ++t)
+          u[t] = k + 1 + h + t < w ? T[o + k][o + k + 1 + h + t] : 0.0;
 #pragma unroll
-        for(int i = 0; i < kW / 4; ++i)
-          if(h + i < kW - 1) s[kW - 1 - h - i] = fma(-u[i], x, s[kW - 2 - h - i]);
+        for(int t = 0; t < kW / 4; ++t)
+          if(h + t < kW - 1) s[h + t] = fma(-u[t], x, s[h + t + 1]);
       }
-      T[o + k][o + lane] = x;
+      T[o + lane][o + k] = x;
     }
   }
 }
@@ -280,26 +285,26 @@ HPLB_DEV void product32(double (&acc)[4], const double* A, const double* B) {
   }
 }
 
-// In-place inverse of the upper triangular kTb x kTb block T (the identity from row
-// and column kb on): both 32 x 32 halves by a warp each, joined by
-// X12 = -X11 (U12 X22), W (32 rows) between.  Every panel of hplb_getrs waits for one
-// of these, the transposed solve for two: kTb steps with two block barriers and a
-// division each (invert_upper) take about 17 us longer (N = 1000, NB = 64, 32
-// right-hand sides, plain 721 us, now 419; transposed 2.16 ms, now 1.59).
+// In-place inverse of the upper triangular kTb x kTb block T (the identity from row and
+// column kb on): both 32 x 32 halves by a warp each, joined (of a unit-lower L's
+// transpose left as they are) by X12 = -(X11 U12) X22, W (32 rows) between.  Every panel of hplb_getrs waits for one of these, the transposed
+// solve for two: kTb steps with two block barriers and a division each (invert_upper)
+// take about 17 us longer (N = 1000, NB = 64, 32 right-hand sides, plain 721 us, now
+// 419; transposed 2.16 ms, now 1.59).
 template <bool UNIT>
 HPLB_DEV void invert_upper_halves(double (*T)[kTp], double (*W)[kTp], int kb) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if(warp == 0) invert_upper32<UNIT>(T, 0, min(32, kb));
   if(warp == 1 && kb > 32) invert_upper32<UNIT>(T, 32, kb - 32);
-  if(kb <= 32) return;  // U12 is 0
+  if(UNIT || kb <= 32) return;  // (U12 is 0)
   const int r = (warp & 1) * 16 + (lane >> 2), c = (warp >> 1) * 8 + 2 * (lane & 3);
   double    acc[4];
   __syncthreads();
-  product32(acc, &T[0][32], &T[32][32]);
+  product32(acc, &T[0][0], &T[0][32]);
 #pragma unroll
   for(int e = 0; e < 4; ++e) W[r + (e >> 1) * 8][c + (e & 1)] = acc[e];
   __syncthreads();
-  product32(acc, &T[0][0], &W[0][0]);
+  product32(acc, &W[0][0], &T[32][32]);
 #pragma unroll
   for(int e = 0; e < 4; ++e) T[r + (e >> 1) * 8][32 + c + (e & 1)] = -acc[e];
 }
@@ -414,8 +419,8 @@ trsm_kernel(const double* __restrict__ A, int64_t ld, int ns, int rows, int nrhs
     for(int e = 0; e < 4; ++e) {
       const int r = rt + g + (e >> 1) * 8, q = 2 * t4 + (e & 1);
       y[e] -= acc[e] + S.X[1][q][r];
-      S.X[0][q][r] = y[e];
-      bad |= !isfinite(y[e]);
+      S.X[0][q][r] = r < kb ? y[e] : 0.0;
+      bad |= r < kb && !isfinite(y[e]);
     }
   }
   if(!solve) {
@@ -427,37 +432,67 @@ trsm_kernel(const double* __restrict__ A, int64_t ld, int ns, int rows, int nrhs
       }
     return;
   }
-  if(__syncthreads_or(bad)) {
-    // x = D^-1 (y - sum) over D^-1's triangle alone: an infinity or NaN in y reaches
-    // only the rows that depend on it, which the full products below would not keep.
+  if(LOWER) {
+    // x = L^-1 (y - sum) by the halves of 32 rows, each with its own inverse: the
+    // inverse of all 64 would multiply the first half's rounding by the second's
+    // (|A^T x - b| 1.15 to 1.23 times as large, N = 128 to 700, NB = 64 to 256).
+    auto times = [&](double (&x)[4], const double (*v)[kTp], int k0) {
+#pragma unroll
+      for(int s = 0; s < 32; s += 8) {
+        const int    k = k0 + s + t4, r = rt + g;
+        const double a[4] = {S.T[k][r], S.T[k][r + 8], S.T[k + 4][r], S.T[k + 4][r + 8]};
+        const double w[2] = {v[g][k], v[g][k + 4]};
+        dmma(x, a, w);
+      }
+    };
+    const bool top = kh == 0 && rt < 32, bottom = kh == 0 && rt >= 32;
+    double     x[4] = {0.0, 0.0, 0.0, 0.0}, z[4] = {0.0, 0.0, 0.0, 0.0};
+    __syncthreads();
+    if(top) {
+      times(x, S.X[0], 0);
+#pragma unroll
+      for(int e = 0; e < 4; ++e) S.X[1][2 * t4 + (e & 1)][rt + g + (e >> 1) * 8] = x[e];
+    }
+    if(kb > 32) {
+      __syncthreads();
+      if(bottom) {
+        times(z, S.X[1], 0);
+#pragma unroll
+        for(int e = 0; e < 4; ++e) {
+          const int r = rt + g + (e >> 1) * 8;
+          S.X[0][2 * t4 + (e & 1)][r] = r < kb ? y[e] - z[e] : 0.0;
+        }
+      }
+      __syncthreads();
+      if(bottom) times(x, S.X[0], 32);
+    }
+    if(kh == 0) {
+#pragma unroll
+      for(int e = 0; e < 4; ++e) {
+        const int r = rt + g + (e >> 1) * 8, q = 2 * t4 + (e & 1);
+        if(r < kb && q < nq) X[(size_t)(r0 + r) + (size_t)(q0 + q) * (size_t)ldx] = x[e];
+      }
+      __threadfence();
+    }
+  } else if(__syncthreads_or(bad)) {
+    // x = U^-1 (y - sum) over the triangle alone: an infinity or NaN in y reaches only
+    // the rows that depend on it, which the full products below would not keep.
     if(kh == 0) {
       for(int e = 0; e < 4; ++e) {
         const int r = rt + g + (e >> 1) * 8, q = 2 * t4 + (e & 1);
         if(r >= kb || q >= nq) continue;
         double x = 0.0;
-        for(int k = LOWER ? 0 : r; k < (LOWER ? r + 1 : kb); ++k)
-          x = fma(LOWER ? S.T[k][r] : S.T[r][k], S.X[0][q][k], x);
+        for(int k = r; k < kb; ++k) x = fma(S.T[r][k], S.X[0][q][k], x);
         X[(size_t)(r0 + r) + (size_t)(q0 + q) * (size_t)ldx] = x;
       }
       __threadfence();
     }
-  } else if(kh == 0) {  // x = D^-1 (y - sum), two chains
+  } else if(kh == 0) {  // x = U^-1 (y - sum), two chains
     double x0[4] = {0.0, 0.0, 0.0, 0.0}, x1[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for(int s = 0; s < kTb; s += 8) {
-      const int k = s + t4, r = rt + g;
-      double    a[4];
-      if(LOWER) {
-        a[0] = S.T[k][r];
-        a[1] = S.T[k][r + 8];
-        a[2] = S.T[k + 4][r];
-        a[3] = S.T[k + 4][r + 8];
-      } else {
-        a[0] = S.T[r][k];
-        a[1] = S.T[r + 8][k];
-        a[2] = S.T[r][k + 4];
-        a[3] = S.T[r + 8][k + 4];
-      }
+      const int    k = s + t4, r = rt + g;
+      const double a[4] = {S.T[r][k], S.T[r + 8][k], S.T[r][k + 4], S.T[r + 8][k + 4]};
       const double v[2] = {S.X[0][g][k], S.X[0][g][k + 4]};
       if(s & 8)
         dmma(x1, a, v);

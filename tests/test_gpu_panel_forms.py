@@ -257,6 +257,33 @@ def test_trsm_upper_block_edges(hlib, n, nrhs):
     assert np.all(np.abs(U @ X - B) <= bound)
 
 
+@pytest.mark.parametrize("n,nb", [(200, 64), (400, 128)])
+def test_transposed_getrs_residual_of_the_block_solve(hlib, oracle, n, nb):
+    """|A^T x - b| of random systems against LAPACK's, in the geometric mean over 24 of
+    them.  With unit-lower blocks applied as two inverses of 32 rows, as the blocked
+    substitution does, 1.15 and 1.11 times LAPACK's; with one inverse of 64 rows 1.40
+    and 1.28.  The logarithms spread by about 0.3 (0.06 in the mean)."""
+    import torch
+
+    from rochpl_b200.hpl import Algo
+
+    logs = []
+    for seed in range(24):
+        g = np.random.default_rng(seed)
+        A, B = g.random((n, n)) - 0.5, g.random((n, 3)) - 0.5
+        LU = torch.from_numpy(np.ascontiguousarray(A.T)).cuda()
+        X = torch.from_numpy(np.ascontiguousarray(B.T)).cuda()
+        piv = torch.zeros(n, dtype=torch.int32, device="cuda")
+        assert hlib.getrf(Algo(nb, 32, 2, 2, 2, 1, 0).c(), n, LU.data_ptr(), n,
+                          piv.data_ptr()) == 0
+        hlib.getrs(1, n, nb, 3, LU.data_ptr(), n, piv.data_ptr(), X.data_ptr(), n)
+        M, ml = A.T, A.T.astype(np.longdouble)
+        ours, ref = (np.linalg.norm((ml @ x - B).astype(float)) / np.linalg.norm(x)
+                     for x in (X.cpu().numpy().T, np.linalg.solve(M, B)))
+        logs.append(np.log(ours / ref))
+    assert np.exp(np.mean(logs)) <= 1.25
+
+
 @pytest.mark.parametrize("n,row", [(40, 7), (64, 33), (100, 70), (200, 90)])
 @pytest.mark.parametrize("bad", [np.inf, np.nan])
 def test_trsm_upper_non_finite_rows(hlib, n, row, bad):
