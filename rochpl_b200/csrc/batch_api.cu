@@ -20,7 +20,12 @@ static const int kClassUpper[HPLB_BATCH_CLASSES] = {48, 96, 192, 384, 768, INT_M
 // The built-in table is what the tuner picks on B200 for 1 to 16 right-hand
 // sides (ms per batch of 296 systems, one right-hand side, width 16 -> this
 // table: n = 40 0.19 -> 0.165, 80 0.375 -> 0.331, 160 0.97 -> 0.80, 320 3.44 ->
-// 2.64, 640 18.2 -> 10.7, 1024 53 -> 28.5).
+// 2.64, 640 18.2 -> 10.7, 1024 53 -> 28.5), and it is the faster one for more as well
+// (64 and 300 right-hand sides: 600 systems of 16 to 96 rows 0.69 -> 0.53 and 1.72 ->
+// 1.32, 150 of 64 to 512 4.5 -> 3.0 and 9.6 -> 5.7, 600 of 32 to 1024 25 -> 14 and
+// 47 -> 21; stored-factor solves 1.1 to 1.5 times as fast).  |A x - b| / (eps |A| |x|)
+// is LAPACK's: n = 320 2.2, 640 3.7, LAPACK 2.1 and 3.7; 16-wide panels, which
+// subtract their products one panel at a time, 1.4 and 1.9.
 static const int kDefaultNb[HPLB_BATCH_CLASSES]  = {32, 32, 32, HPLB_BATCH_RECURSIVE,
                                                     HPLB_BATCH_RECURSIVE, HPLB_BATCH_RECURSIVE};
 static const int kTuneN[HPLB_BATCH_CLASSES]      = {40, 80, 160, 320, 640, 1024};

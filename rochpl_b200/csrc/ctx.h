@@ -55,7 +55,7 @@ struct hplb_ctx {
   // Multi-RHS solve workspaces (hplb_getrs).
   double* r_t    = nullptr;  size_t r_t_cap    = 0;  // transposed factors (trans = 1)
   double* r_ws   = nullptr;  size_t r_ws_cap   = 0;  // block copies and inverses
-  int*    r_perm = nullptr;  size_t r_perm_cap = 0;  // one panel's row map
+  int*    r_perm = nullptr;  size_t r_perm_cap = 0;  // every panel's row map
 
   int          leaf_kind = HPLB_LEAF_AUTO;  // hplb_set_option(HPLB_OPT_LEAF)
   int          panel_sms = HPLB_PANEL_SMS_AUTO;  // hplb_set_option(HPLB_OPT_PANEL_SMS)

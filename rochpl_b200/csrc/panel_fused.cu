@@ -1,4 +1,4 @@
-// A whole panel in one launch: the recursive factorisation of an M x NB panel
+// A whole panel in a few launches: the recursive factorisation of an M x NB panel
 // (HPL_pdrpanrlT / HPL_pdrpanllT / HPL_pdrpancrT, src/pfact/HPL_pdrpanrlT.cpp:74-160),
 // its interchanges, the row map and L11^-1, on ONE thread-block cluster of up
 // to 16 CTAs that walks a list of operations made by the host's recursion.
