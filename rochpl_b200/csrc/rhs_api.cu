@@ -11,13 +11,12 @@
 // and
 //   A^-T = P_0^T E_0^T ... P_{np-1}^T E_{np-1}^T U^-T.
 // Up to 128 right-hand sides a panel's L11 and the rows below it take one
-// persistent launch (launch_trsm_lower): with a CTA per column for
-// L11 and a product kernel for the rows below, the chain of launches bounded the
-// solve (N = 8192, NB = 512, 32 right-hand sides: 4.25 ms, now 1.69).  More
-// right-hand sides take the blocked substitution and DMMA GEMMs (explicit
-// inverses of 512 x 512 blocks would cost far more).  The row maps of all panels
-// come from one launch; the transposed solve reads a transposed copy of the factors so that
-// its GEMMs are plain NN.
+// persistent launch (launch_trsm_lower): with a CTA per column for L11 and a product
+// kernel for the rows below, the chain of launches bounded the solve (N = 8192,
+// NB = 512, 32 right-hand sides: 4.25 ms, now 1.40).  More right-hand sides take the
+// blocked substitution and DMMA GEMMs (explicit inverses of 512 x 512 blocks would
+// cost far more).  The row maps of all panels come from one launch; the transposed
+// solve reads a transposed copy of the factors so that its GEMMs are plain NN.
 #include <algorithm>
 
 #include "ctx.h"

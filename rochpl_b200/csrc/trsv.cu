@@ -200,7 +200,7 @@ trsv_kernel(const double* __restrict__ A, int64_t ld, int n, const double* __res
 // 12.3 us per row block (N = 8192: 1576 us, now 424 us).  Up to 128 right-hand sides
 // run in one launch, their groups' chains beside each other; a launch per 32 was as
 // many chains in turn (hplb_getrs, 64 right-hand sides, N = 1000, NB = 64: plain 1.30,
-// transposed 3.20 ms, now 0.73 and 2.16).  Waits are bounded (status site 42).  X may
+// transposed 3.20 ms; one launch 0.73 and 2.16).  Waits are bounded (status site 42).  X may
 // alias Y: a block of Y is read only by its own CTA, before that CTA writes X there.
 constexpr int kNr       = 128;      // right-hand sides per launch
 constexpr int kNg       = 8;        // right-hand sides per CTA
